@@ -16,6 +16,7 @@
 
 #include "sc_fft.cuh"
 #include "sc_internal.h"
+#include "sc_sweep_sizes.h"
 #include "sc_les.h"
 #include "sc_cnn.h"
 #include "sc_cnn_cc.h"
@@ -190,8 +191,8 @@ void plan_free(sc_plan* p) {
   if (p->cap) cudaStreamDestroy(p->cap);
 }
 
-// Host image of a twiddle buffer: exp(-2 pi i m / n) from long double, and for
-// FP32 n = 810 the x sweep's pair table after it (sc::twiddle_buffer_bytes).
+// Host image of a twiddle buffer (sc::twiddle_buffer_bytes): exp(-2 pi i m / n)
+// from long double, and the tables made from it.
 template <typename R>
 std::vector<unsigned char> twiddle_image(int n) {
   using C = typename sc::V2<R>::T;
@@ -203,8 +204,16 @@ std::vector<unsigned char> twiddle_image(int n) {
     h[m].x = (R)cosl(th);
     h[m].y = (R)(-sinl(th));
   }
-  if (img.size() > sizeof(C) * (size_t)n)
+  if (sc::twiddle_x_offset(n, sizeof(C)) > sizeof(C) * (size_t)n)
     sc::xpair810_twiddles(reinterpret_cast<const float2*>(h), reinterpret_cast<float*>(h + n));
+  int n1 = 0, n2 = 0;
+  if (sc::sweep_size(n, sizeof(R) == 4, &n1, &n2)) {
+    C* t1 = reinterpret_cast<C*>(img.data() + sc::twiddle_x_offset(n, sizeof(C)));
+    for (int q = 0; q < n; ++q) {
+      t1[q] = h[(q / n2) * (q % n2)];
+      t1[n + q] = h[(q / n1) * (q % n1)];
+    }
+  }
   return img;
 }
 
@@ -277,7 +286,7 @@ int even_up(int k) { return k + (k & 1); }
 // (x extent kout+1, y/z extent 2 kout+1) in `sig` (default: the plan's).
 template <typename R>
 int products(sc_plan* p, void* const* u, cudaStream_t st, cudaEvent_t* ev = nullptr, int kout = -1,
-             void* const* sig = nullptr) {
+             void* const* sig = nullptr, bool pinned = false) {
   const int n = p->n, K1 = p->K1, K2 = p->K2, kc = p->kc;
   if (kout < 0) kout = kc;
   if (!sig) sig = p->sig;
@@ -308,7 +317,7 @@ int products(sc_plan* p, void* const* u, cudaStream_t st, cudaEvent_t* ev = null
     for (int c = 0; c < 6; ++c) x.out[c] = p->dd[c];
     x.D = 3; x.K1in = K1; x.K1out = K1o; x.nrows = (long long)n * n; x.scale = 1.0 / ((double)n * n * n);
     x.ldo = ldo;
-    x.variant = p->variant[2];
+    x.variant = pinned ? 1 : p->variant[2];
     sc::launch_xsweep_ns<R>(n, x, p->tw, st);
     mark();
     sc::ColArgs f = y_forward_args(K1o, n, kout, ldo);
@@ -353,7 +362,7 @@ int products(sc_plan* p, void* const* u, cudaStream_t st, cudaEvent_t* ev = null
 // ---------------------------------------------------------------------------
 template <typename R>
 int c2p_batch(sc_plan* p, void* const* bb, void* const* cb, void* const* in, void* const* out, int m,
-              cudaStream_t st) {
+              cudaStream_t st, bool pinned = false) {
   const int n = p->n, K1 = p->K1, K2 = p->K2, kc = p->kc;
   for (int c0 = 0; c0 < m; c0 += 12) {
     const int mc = m - c0 < 12 ? m - c0 : 12;
@@ -377,6 +386,7 @@ int c2p_batch(sc_plan* p, void* const* bb, void* const* cb, void* const* in, voi
     sc::XPlainArgs x{};
     for (int c = 0; c < mc; ++c) { x.in[c] = cb[c]; x.out[c] = out[c0 + c]; }
     x.ncomp = mc; x.K1 = K1; x.nrows = p->D == 3 ? (long long)n * n : n; x.scale = 1.0;
+    x.pinned = pinned;
     sc::launch_x_c2r<R>(n, x, p->tw, st);
   }
   return check_launch("compact to physical");
@@ -384,7 +394,7 @@ int c2p_batch(sc_plan* p, void* const* bb, void* const* cb, void* const* in, voi
 
 template <typename R>
 int p2c_batch(sc_plan* p, void* const* bb, void* const* cb, void* const* in, void* const* out, int m,
-              cudaStream_t st) {
+              cudaStream_t st, bool pinned = false) {
   const int n = p->n, K1 = p->K1, K2 = p->K2, kc = p->kc;
   for (int c0 = 0; c0 < m; c0 += 12) {
     const int mc = m - c0 < 12 ? m - c0 : 12;
@@ -392,6 +402,7 @@ int p2c_batch(sc_plan* p, void* const* bb, void* const* cb, void* const* in, voi
     for (int c = 0; c < mc; ++c) { x.in[c] = in[c0 + c]; x.out[c] = cb[c]; }
     x.ncomp = mc; x.K1 = K1; x.nrows = p->D == 3 ? (long long)n * n : n;
     x.scale = 1.0 / std::pow((double)n, p->D);
+    x.pinned = pinned;
     sc::launch_x_r2c<R>(n, x, p->tw, st);
     sc::ColArgs f{};
     if (p->D == 3) {
@@ -520,6 +531,10 @@ sc::MlpArgs mlp_args(sc_closure* cl, const void* const* G, void* const* tau) {
   a.mode = cl->kind == sc::kTbnn ? 1 : 0;
   return a;
 }
+
+// Right-hand sides with the one-pass BF16 network keep the x kernels their
+// results were made with (sc_fast.cu says why).
+bool pinned(const sc_closure* cl) { return cl && cl->kind == sc::kCnn && !cl->cnn_split; }
 
 // The split-precision fields of a forward pass (pre[] as the caller set it).
 void tc_split_args(const sc_closure* cl, sc::CnnArgs& a) {
@@ -696,7 +711,7 @@ int closure_tauhat(sc_closure* cl, void* const* u, cudaStream_t st, void* const*
     if (tau_phys_out) return c2p_batch<R>(p, cl->bb, cl->cb, cl->th, tau_phys_out, NP, st);
     return check_launch("dynamic Smagorinsky");
   } else if (cl->kind == sc::kCnn) {
-    if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, u, cl->gp, D, st))) return rc;  // u (physical)
+    if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, u, cl->gp, D, st, pinned(cl)))) return rc;  // u (physical)
     SC_CU(cudaMemsetAsync(cl->dsum, 0, sizeof(double), st));
     sc::launch_spectral_energy<R>(u, D, D, p->n, p->K1, p->K2, 1, p->kc, 2.0 * M_PI / p->l, 1, cl->dsum, st);
     sc::CnnArgs a{};
@@ -742,7 +757,7 @@ int closure_tauhat(sc_closure* cl, void* const* u, cudaStream_t st, void* const*
                             cudaMemcpyDeviceToDevice, st));
     return check_launch("closure");
   }
-  return p2c_batch<R>(p, cl->bb, cl->cb, cl->tp, cl->th, NP, st);
+  return p2c_batch<R>(p, cl->bb, cl->cb, cl->tp, cl->th, NP, st, pinned(cl));
 }
 
 template <typename R>
@@ -765,7 +780,7 @@ void add_closure_stress(sc::EpiArgs& e, sc_closure* cl, int D) {
 
 template <typename R>
 int stage_rhs(sc_plan* p, sc_closure* cl, void* const* us, cudaStream_t st) {
-  int rc = products<R>(p, us, st);
+  int rc = products<R>(p, us, st, nullptr, -1, nullptr, pinned(cl));
   if (rc) return rc;
   if (cl && cl->kind != sc::kNoClosure) return closure_tauhat<R>(cl, us, st);
   return SC_OK;
@@ -1298,7 +1313,8 @@ int microbench_impl(int kernel, int n, long long count, int reps, double* ms, do
     ca.out[0] = alloc(kernel == 3 ? mid : cube);
     ca.ncomp = 1; ca.ncols = (int)count;
     b = (double)esz * K1 * count * (K2 + n);
-  } else if (kernel == 2) {  // 3D x sweep over `count` rows
+  } else if (kernel == 2) {  // 3D x sweep over `count` rows (whole row pairs)
+    count += count & 1;
     for (int c = 0; c < 3; ++c) xa.in[c] = alloc((size_t)K1 * count);
     for (int c = 0; c < 6; ++c) xa.out[c] = alloc((size_t)K1 * count);
     xa.D = 3; xa.K1in = K1; xa.K1out = K1; xa.nrows = count; xa.scale = 1.0 / ((double)n * n * n);
@@ -1964,7 +1980,7 @@ int vmax_impl(sc_plan* p, void* const* uc, double* vmax, cudaStream_t st) {
   double h = 0;
   SC_CU(cudaMemcpyAsync(&h, p->dscal + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
   SC_CU(cudaStreamSynchronize(st));
-  *vmax = h;
+  *vmax = std::sqrt(h);  // the square root is monotone: one here instead of one per point
   return SC_OK;
 }
 

@@ -155,369 +155,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
-// x sweep with the Navier-Stokes products (rows are contiguous)
-// ---------------------------------------------------------------------------
-template <int N> struct X2Rows;
-template <> struct X2Rows<810> { static constexpr int TR = 2; };
-template <> struct X2Rows<256> { static constexpr int TR = 4; };
-template <> struct X2Rows<128> { static constexpr int TR = 8; };
-template <> struct X2Rows<64> { static constexpr int TR = 16; };
-
-template <int N, int D> struct X2Cfg {
-  static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, N2P = N2 + 1;
-  static constexpr int TR = X2Rows<N>::TR;
-  static constexpr int K1M = N / 3 + 1;           // widest input row (2/3-truncated spectrum)
-  static constexpr int NPI = D == 3 ? 2 * TR : TR;   // inverse pencils
-  static constexpr int NPF = D == 3 ? 3 * TR : 2 * TR;  // forward pencils
-  static constexpr int NT = 192;
-  static constexpr size_t RIN = size_t(D) * TR * K1M * sizeof(float2);
-  static constexpr size_t UPH = size_t(D) * TR * N * sizeof(float);
-  static constexpr size_t ZB = size_t(NPF) * (2 * K1M - 1) * sizeof(float2);
-  static constexpr size_t A0 = (RIN + UPH) > ZB ? (RIN + UPH) : ZB;  // Rin+U, later aliased by Z
-  static constexpr size_t YB = size_t(NPF) * N1 * N2P * sizeof(float2);
-  static constexpr size_t SMEM = A0 + YB;
-};
-
-template <int N> __device__ __forceinline__ float2 hext2(const float2* row, int K1, int f) {
-  const int kmax = K1 - 1;
-  if (f == 0) return make_float2(row[0].x, 0.f);
-  if (f <= kmax) return row[f];
-  if (f >= N - kmax) { const float2 v = row[N - f]; return make_float2(v.x, -v.y); }
-  return make_float2(0.f, 0.f);
-}
-
-template <int N, int D>
-__global__ void __launch_bounds__(X2Cfg<N, D>::NT)
-k_xsweep2(const XArgs a, const float2* __restrict__ tw) {
-  using C = float2;
-  using Cfg = X2Cfg<N, D>;
-  constexpr int N1 = Cfg::N1, N2 = Cfg::N2, N2P = Cfg::N2P, TR = Cfg::TR, K1M = Cfg::K1M;
-  constexpr int NPI = Cfg::NPI, NPF = Cfg::NPF, NT = Cfg::NT;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* rin = reinterpret_cast<C*>(smem_raw);                        // [D][TR][K1M]
-  float* uph = reinterpret_cast<float*>(smem_raw + Cfg::RIN);     // [D][TR][N]
-  C* zb = reinterpret_cast<C*>(smem_raw);                         // [NPF][2*K1M-1] (after F1)
-  C* yb = reinterpret_cast<C*>(smem_raw + Cfg::A0);               // [NPF][N1][N2P]
-  const long long row0 = (long long)blockIdx.x * TR;
-  const int K1 = a.K1in;
-  const int ko = a.K1out - 1;
-  constexpr int ZS = 2 * K1M - 1;
-
-  // L: stage the TR spectral rows of each component (contiguous in global memory)
-  {
-    constexpr int TOT = D * TR * K1M;
-    constexpr int LPT = (TOT + NT - 1) / NT;
-    // select the component pointer instead of indexing the parameter array at run time
-    const C* in0 = static_cast<const C*>(a.in[0]);
-    const C* in1 = static_cast<const C*>(a.in[1]);
-    const C* in2 = static_cast<const C*>(a.in[D == 3 ? 2 : 1]);
-    C v[LPT];
-#pragma unroll
-    for (int i = 0; i < LPT; ++i) {
-      const int idx = threadIdx.x + i * NT;
-      v[i] = make_float2(0.f, 0.f);
-      const int cmp = idx / (TR * K1M), r = (idx / K1M) % TR, kx = idx % K1M;
-      if (idx < TOT && kx < K1 && row0 + r < a.nrows)
-        v[i] = __ldg((cmp == 0 ? in0 : cmp == 1 ? in1 : in2) + (row0 + r) * K1 + kx);
-    }
-#pragma unroll
-    for (int i = 0; i < LPT; ++i) {
-      const int idx = threadIdx.x + i * NT;
-      if (idx < TOT) rin[idx] = v[i];
-    }
-  }
-  __syncthreads();
-
-  // I1: inverse step 1 (pencil p: row p % TR; kind 0: u1 + i u2, kind 1: u3)
-  for (int it = threadIdx.x; it < NPI * N2; it += NT) {
-    const int p = it / N2, j = it % N2;
-    const int r = p % TR, kind = p / TR;
-    C v[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-      const int f = N2 * n1 + j;
-      if (kind == 0) {
-        const C x1 = hext2<N>(rin + (0 * TR + r) * K1M, K1, f);
-        const C x2 = hext2<N>(rin + (1 * TR + r) * K1M, K1, f);
-        v[n1] = make_float2(x1.x - x2.y, x1.y + x2.x);
-      } else {
-        v[n1] = hext2<N>(rin + (2 * TR + r) * K1M, K1, f);
-      }
-    }
-    DFT<N1, true, C>::run(v);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1) {
-      const C w = __ldg(&tw[j * k1]);
-      v[k1] = cmul(v[k1], make_float2(w.x, -w.y));
-    }
-    C* yp = yb + p * N1 * N2P;
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) yp[k1 * N2P + j] = v[k1];
-  }
-  __syncthreads();
-
-  // I2: inverse step 2 -> physical velocities at x = i + N1 k2
-  for (int it = threadIdx.x; it < NPI * N1; it += NT) {
-    const int p = it / N1, i = it % N1;
-    const int r = p % TR, kind = p / TR;
-    C w[N2];
-    const C* yp = yb + p * N1 * N2P + i * N2P;
-#pragma unroll
-    for (int n2 = 0; n2 < N2; ++n2) w[n2] = yp[n2];
-    DFT<N2, true, C>::run(w);
-    if (kind == 0) {
-      float* u1 = uph + (0 * TR + r) * N;
-      float* u2 = uph + (1 * TR + r) * N;
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) { u1[i + N1 * k2] = w[k2].x; u2[i + N1 * k2] = w[k2].y; }
-    } else {
-      float* u3 = uph + (2 * TR + r) * N;
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) u3[i + N1 * k2] = w[k2].x;
-    }
-  }
-  __syncthreads();
-
-  // F1: products (scaled) and forward step 1
-  const float sc = float(a.scale);
-  for (int it = threadIdx.x; it < NPF * N2; it += NT) {
-    const int p = it / N2, j = it % N2;
-    const int r = p % TR, kind = p / TR;
-    const float* u1 = uph + (0 * TR + r) * N;
-    const float* u2 = uph + (1 * TR + r) * N;
-    const float* u3 = uph + ((D == 3 ? 2 : 0) * TR + r) * N;
-    C v[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-      const int x = N2 * n1 + j;
-      const float a1 = u1[x], a2 = u2[x];
-      if (D == 3) {
-        const float a3 = u3[x];
-        v[n1] = kind == 0 ? make_float2(a1 * a1 * sc, a2 * a2 * sc)
-              : kind == 1 ? make_float2(a3 * a3 * sc, a1 * a2 * sc)
-                          : make_float2(a2 * a3 * sc, a3 * a1 * sc);
-      } else {
-        v[n1] = kind == 0 ? make_float2(a1 * a1 * sc, a2 * a2 * sc) : make_float2(a1 * a2 * sc, 0.f);
-      }
-    }
-    DFT<N1, false, C>::run(v);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1) v[k1] = cmul(v[k1], __ldg(&tw[j * k1]));
-    C* yp = yb + p * N1 * N2P;
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) yp[k1 * N2P + j] = v[k1];
-  }
-  __syncthreads();
-
-  // F2: forward step 2, keep X[k] for k <= ko and k >= N - ko
-  for (int it = threadIdx.x; it < NPF * N1; it += NT) {
-    const int p = it / N1, i = it % N1;
-    C w[N2];
-    const C* yp = yb + p * N1 * N2P + i * N2P;
-#pragma unroll
-    for (int n2 = 0; n2 < N2; ++n2) w[n2] = yp[n2];
-    DFT<N2, false, C>::run(w);
-    C* zp = zb + p * ZS;
-#pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) {
-      const int k = i + N1 * k2;
-      if (k <= ko) zp[k] = w[k2];
-      else if (k >= N - ko) zp[ko + (N - k)] = w[k2];
-    }
-  }
-  __syncthreads();
-
-  // S: split the paired spectra and store the product rows
-  constexpr int NBF = NPF / TR;
-  const int K1o = a.K1out;
-  const long long ldo = a.ldo > 0 ? a.ldo : K1o;
-  for (int it = threadIdx.x; it < TR * K1o; it += NT) {
-    const int r = it / K1o, kx = it % K1o;
-    const long long row = row0 + r;
-    if (row >= a.nrows) continue;
-#pragma unroll
-    for (int b = 0; b < NBF; ++b) {
-      const C* zp = zb + (b * TR + r) * ZS;
-      const C z = zp[kx], zc = zp[kx == 0 ? 0 : ko + kx];
-      const C xa = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
-      const C xbv = make_float2(0.5f * (z.y + zc.y), 0.5f * (zc.x - z.x));
-      static_cast<C*>(a.out[2 * b])[row * ldo + kx] = xa;
-      if (2 * b + 1 < (D == 3 ? 6 : 3)) static_cast<C*>(a.out[2 * b + 1])[row * ldo + kx] = xbv;
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// 3D x sweep, rows paired: u3 of rows 2q and 2q+1 share one inverse transform
-// (1.5 inverse transforms per row instead of 2) and the forward side runs in
-// two halves of TR/2 rows so that every phase keeps ~90 % of the threads busy.
-// ---------------------------------------------------------------------------
-template <int N> struct X3Rows;
-template <> struct X3Rows<810> { static constexpr int TR = 4; };
-template <> struct X3Rows<256> { static constexpr int TR = 8; };
-template <> struct X3Rows<128> { static constexpr int TR = 16; };
-template <> struct X3Rows<64> { static constexpr int TR = 32; };
-
-template <int N> struct X3Cfg {
-  static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, N2P = N2 + 1;
-  static constexpr int TR = X3Rows<N>::TR, TH = TR / 2;
-  static constexpr int K1M = N / 3 + 1;
-  static constexpr int NPI = TR + TH;   // inverse pencils: u1 + i u2 per row, u3 pairs
-  static constexpr int NPF = 3 * TH;    // forward pencils of one half
-  static constexpr int NT = 192;
-  static constexpr size_t RIN = size_t(3) * TR * K1M * sizeof(float2);
-  static constexpr size_t ZB = size_t(NPF) * (2 * K1M - 1) * sizeof(float2);
-  static constexpr size_t A0 = RIN > ZB ? RIN : ZB;  // Rin, later Z of each half
-  static constexpr size_t UPH = size_t(3) * TR * N * sizeof(float);
-  static constexpr int NPY = NPI > NPF ? NPI : NPF;
-  static constexpr size_t YB = size_t(NPY) * N1 * N2P * sizeof(float2);
-  static constexpr size_t SMEM = A0 + UPH + YB;
-};
-
-template <int N>
-__global__ void __launch_bounds__(X3Cfg<N>::NT)
-k_xsweep3(const XArgs a, const float2* __restrict__ tw) {
-  using C = float2;
-  using Cfg = X3Cfg<N>;
-  constexpr int N1 = Cfg::N1, N2 = Cfg::N2, N2P = Cfg::N2P, TR = Cfg::TR, TH = Cfg::TH, K1M = Cfg::K1M;
-  constexpr int NPI = Cfg::NPI, NPF = Cfg::NPF, NT = Cfg::NT;
-  constexpr int ZS = 2 * K1M - 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* rin = reinterpret_cast<C*>(smem_raw);                         // [3][TR][K1M]
-  C* zb = reinterpret_cast<C*>(smem_raw);                          // [NPF][ZS] after I1
-  float* uph = reinterpret_cast<float*>(smem_raw + Cfg::A0);       // [3][TR][N]
-  C* yb = reinterpret_cast<C*>(smem_raw + Cfg::A0 + Cfg::UPH);     // [NPY][N1][N2P]
-  const long long row0 = (long long)blockIdx.x * TR;
-  const int K1 = a.K1in;
-  const int ko = a.K1out - 1;
-  {
-    constexpr int TOT = 3 * TR * K1M;
-    constexpr int LPT = (TOT + NT - 1) / NT;
-    // select the component pointer instead of indexing the parameter array at run time
-    const C* in0 = static_cast<const C*>(a.in[0]);
-    const C* in1 = static_cast<const C*>(a.in[1]);
-    const C* in2 = static_cast<const C*>(a.in[2]);
-    C v[LPT];
-#pragma unroll
-    for (int i = 0; i < LPT; ++i) {
-      const int idx = threadIdx.x + i * NT;
-      v[i] = make_float2(0.f, 0.f);
-      const int cmp = idx / (TR * K1M), r = (idx / K1M) % TR, kx = idx % K1M;
-      if (idx < TOT && kx < K1 && row0 + r < a.nrows)
-        v[i] = __ldg((cmp == 0 ? in0 : cmp == 1 ? in1 : in2) + (row0 + r) * K1 + kx);
-    }
-#pragma unroll
-    for (int i = 0; i < LPT; ++i) {
-      const int idx = threadIdx.x + i * NT;
-      if (idx < TOT) rin[idx] = v[i];
-    }
-  }
-  __syncthreads();
-  // I1: pencils p < TR: u1 + i u2 of row p; p >= TR: u3(row 2q) + i u3(row 2q+1), q = p - TR
-  for (int it = threadIdx.x; it < NPI * N2; it += NT) {
-    const int p = it / N2, j = it % N2;
-    const C* ra;
-    const C* rb;
-    if (p < TR) { ra = rin + (0 * TR + p) * K1M; rb = rin + (1 * TR + p) * K1M; }
-    else { const int q = p - TR; ra = rin + (2 * TR + 2 * q) * K1M; rb = rin + (2 * TR + 2 * q + 1) * K1M; }
-    C v[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-      const int f = N2 * n1 + j;
-      const C x1 = hext2<N>(ra, K1, f), x2 = hext2<N>(rb, K1, f);
-      v[n1] = make_float2(x1.x - x2.y, x1.y + x2.x);
-    }
-    DFT<N1, true, C>::run(v);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1) {
-      const C w = __ldg(&tw[j * k1]);
-      v[k1] = cmul(v[k1], make_float2(w.x, -w.y));
-    }
-    C* yp = yb + p * N1 * N2P;
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) yp[k1 * N2P + j] = v[k1];
-  }
-  __syncthreads();
-  // I2: physical velocities
-  for (int it = threadIdx.x; it < NPI * N1; it += NT) {
-    const int p = it / N1, i = it % N1;
-    C w[N2];
-    const C* yp = yb + p * N1 * N2P + i * N2P;
-#pragma unroll
-    for (int n2 = 0; n2 < N2; ++n2) w[n2] = yp[n2];
-    DFT<N2, true, C>::run(w);
-    float* oa;
-    float* ob;
-    if (p < TR) { oa = uph + (0 * TR + p) * N; ob = uph + (1 * TR + p) * N; }
-    else { const int q = p - TR; oa = uph + (2 * TR + 2 * q) * N; ob = uph + (2 * TR + 2 * q + 1) * N; }
-#pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) { oa[i + N1 * k2] = w[k2].x; ob[i + N1 * k2] = w[k2].y; }
-  }
-  __syncthreads();
-  const float sc = float(a.scale);
-  const int K1o = a.K1out;
-  const long long ldo = a.ldo > 0 ? a.ldo : K1o;
-#pragma unroll 1
-  for (int half = 0; half < 2; ++half) {
-    // F1: products of the half's rows, forward step 1 (pencil p: row half*TH + p % TH, kind p / TH)
-    for (int it = threadIdx.x; it < NPF * N2; it += NT) {
-      const int p = it / N2, j = it % N2;
-      const int r = half * TH + p % TH, kind = p / TH;
-      const float* u1 = uph + (0 * TR + r) * N;
-      const float* u2 = uph + (1 * TR + r) * N;
-      const float* u3 = uph + (2 * TR + r) * N;
-      C v[N1];
-#pragma unroll
-      for (int n1 = 0; n1 < N1; ++n1) {
-        const int x = N2 * n1 + j;
-        const float a1 = u1[x], a2 = u2[x], a3 = u3[x];
-        v[n1] = kind == 0 ? make_float2(a1 * a1 * sc, a2 * a2 * sc)
-              : kind == 1 ? make_float2(a3 * a3 * sc, a1 * a2 * sc)
-                          : make_float2(a2 * a3 * sc, a3 * a1 * sc);
-      }
-      DFT<N1, false, C>::run(v);
-#pragma unroll
-      for (int k1 = 1; k1 < N1; ++k1) v[k1] = cmul(v[k1], __ldg(&tw[j * k1]));
-      C* yp = yb + p * N1 * N2P;
-#pragma unroll
-      for (int k1 = 0; k1 < N1; ++k1) yp[k1 * N2P + j] = v[k1];
-    }
-    __syncthreads();
-    // F2: forward step 2 into Z (the staged input rows are no longer needed)
-    for (int it = threadIdx.x; it < NPF * N1; it += NT) {
-      const int p = it / N1, i = it % N1;
-      C w[N2];
-      const C* yp = yb + p * N1 * N2P + i * N2P;
-#pragma unroll
-      for (int n2 = 0; n2 < N2; ++n2) w[n2] = yp[n2];
-      DFT<N2, false, C>::run(w);
-      C* zp = zb + p * ZS;
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) {
-        const int k = i + N1 * k2;
-        if (k <= ko) zp[k] = w[k2];
-        else if (k >= N - ko) zp[ko + (N - k)] = w[k2];
-      }
-    }
-    __syncthreads();
-    // S: split and store the half's product rows
-    for (int it = threadIdx.x; it < TH * K1o; it += NT) {
-      const int rr = it / K1o, kx = it % K1o;
-      const long long row = row0 + half * TH + rr;
-      if (row >= a.nrows) continue;
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        const C* zp = zb + (b * TH + rr) * ZS;
-        const C z = zp[kx], zc = zp[kx == 0 ? 0 : ko + kx];
-        static_cast<C*>(a.out[2 * b])[row * ldo + kx] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
-        static_cast<C*>(a.out[2 * b + 1])[row * ldo + kx] = make_float2(0.5f * (z.y + zc.y), 0.5f * (zc.x - z.x));
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------------------
 // 3D x sweep for N = 810 = 9 * 9 * 10, one row pair per 96-thread block.
 //
 // Inverse (c2r of the Hermitian-extended rows, k = 9 m1 + m2):
@@ -831,13 +468,192 @@ k_xsweep4(const XArgs a, const float2* __restrict__ tw) {
 }
 
 // ---------------------------------------------------------------------------
-// plain x transforms (to_phys! / to_spec! along x, the closures' and les!'s
-// batches of fields): two-level register FFT per pencil, a pencil being one
-// row of two components packed as a + i b
+// x sweeps around the one-pass BF16 closure network (N = 64 and 128)
 // ---------------------------------------------------------------------------
+// Three layers of BF16 roundings turn any rounding difference of the network's
+// input into a difference of the size of the roundings themselves: the sweeps
+// of sc_xrow.cuh, equally exact, moved the state of a 128^3 step by 1.9e-5
+// where the network's own error is 3.9e-5.  So the transforms of a right-hand
+// side with that network keep these kernels and with them, bit for bit, the
+// results of earlier runs; they cost 70 us of a 2.9 ms step.
+//
+// Product sweep, rows paired: u3 of rows 2q and 2q+1 share one inverse transform
+// (1.5 inverse transforms per row instead of 2) and the forward side runs in two
+// halves of TR/2 rows so that every phase keeps ~90 % of the threads busy.
+template <int N> __device__ __forceinline__ float2 hext2(const float2* row, int K1, int f) {
+  const int kmax = K1 - 1;
+  if (f == 0) return make_float2(row[0].x, 0.f);
+  if (f <= kmax) return row[f];
+  if (f >= N - kmax) { const float2 v = row[N - f]; return make_float2(v.x, -v.y); }
+  return make_float2(0.f, 0.f);
+}
+
+template <int N> struct X3Rows;
+template <> struct X3Rows<128> { static constexpr int TR = 16; };
+template <> struct X3Rows<64> { static constexpr int TR = 32; };
+
+template <int N> struct X3Cfg {
+  static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, N2P = N2 + 1;
+  static constexpr int TR = X3Rows<N>::TR, TH = TR / 2;
+  static constexpr int K1M = N / 3 + 1;
+  static constexpr int NPI = TR + TH;   // inverse pencils: u1 + i u2 per row, u3 pairs
+  static constexpr int NPF = 3 * TH;    // forward pencils of one half
+  static constexpr int NT = 192;
+  static constexpr size_t RIN = size_t(3) * TR * K1M * sizeof(float2);
+  static constexpr size_t ZB = size_t(NPF) * (2 * K1M - 1) * sizeof(float2);
+  static constexpr size_t A0 = RIN > ZB ? RIN : ZB;  // Rin, later Z of each half
+  static constexpr size_t UPH = size_t(3) * TR * N * sizeof(float);
+  static constexpr int NPY = NPI > NPF ? NPI : NPF;
+  static constexpr size_t YB = size_t(NPY) * N1 * N2P * sizeof(float2);
+  static constexpr size_t SMEM = A0 + UPH + YB;
+};
+
+template <int N>
+__global__ void __launch_bounds__(X3Cfg<N>::NT)
+k_xsweep3(const XArgs a, const float2* __restrict__ tw) {
+  using C = float2;
+  using Cfg = X3Cfg<N>;
+  constexpr int N1 = Cfg::N1, N2 = Cfg::N2, N2P = Cfg::N2P, TR = Cfg::TR, TH = Cfg::TH, K1M = Cfg::K1M;
+  constexpr int NPI = Cfg::NPI, NPF = Cfg::NPF, NT = Cfg::NT;
+  constexpr int ZS = 2 * K1M - 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C* rin = reinterpret_cast<C*>(smem_raw);                         // [3][TR][K1M]
+  C* zb = reinterpret_cast<C*>(smem_raw);                          // [NPF][ZS] after I1
+  float* uph = reinterpret_cast<float*>(smem_raw + Cfg::A0);       // [3][TR][N]
+  C* yb = reinterpret_cast<C*>(smem_raw + Cfg::A0 + Cfg::UPH);     // [NPY][N1][N2P]
+  const long long row0 = (long long)blockIdx.x * TR;
+  const int K1 = a.K1in;
+  const int ko = a.K1out - 1;
+  {
+    constexpr int TOT = 3 * TR * K1M;
+    constexpr int LPT = (TOT + NT - 1) / NT;
+    // select the component pointer instead of indexing the parameter array at run time
+    const C* in0 = static_cast<const C*>(a.in[0]);
+    const C* in1 = static_cast<const C*>(a.in[1]);
+    const C* in2 = static_cast<const C*>(a.in[2]);
+    C v[LPT];
+#pragma unroll
+    for (int i = 0; i < LPT; ++i) {
+      const int idx = threadIdx.x + i * NT;
+      v[i] = make_float2(0.f, 0.f);
+      const int cmp = idx / (TR * K1M), r = (idx / K1M) % TR, kx = idx % K1M;
+      if (idx < TOT && kx < K1 && row0 + r < a.nrows)
+        v[i] = __ldg((cmp == 0 ? in0 : cmp == 1 ? in1 : in2) + (row0 + r) * K1 + kx);
+    }
+#pragma unroll
+    for (int i = 0; i < LPT; ++i) {
+      const int idx = threadIdx.x + i * NT;
+      if (idx < TOT) rin[idx] = v[i];
+    }
+  }
+  __syncthreads();
+  // I1: pencils p < TR: u1 + i u2 of row p; p >= TR: u3(row 2q) + i u3(row 2q+1), q = p - TR
+  for (int it = threadIdx.x; it < NPI * N2; it += NT) {
+    const int p = it / N2, j = it % N2;
+    const C* ra;
+    const C* rb;
+    if (p < TR) { ra = rin + (0 * TR + p) * K1M; rb = rin + (1 * TR + p) * K1M; }
+    else { const int q = p - TR; ra = rin + (2 * TR + 2 * q) * K1M; rb = rin + (2 * TR + 2 * q + 1) * K1M; }
+    C v[N1];
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1) {
+      const int f = N2 * n1 + j;
+      const C x1 = hext2<N>(ra, K1, f), x2 = hext2<N>(rb, K1, f);
+      v[n1] = make_float2(x1.x - x2.y, x1.y + x2.x);
+    }
+    DFT<N1, true, C>::run(v);
+#pragma unroll
+    for (int k1 = 1; k1 < N1; ++k1) {
+      const C w = __ldg(&tw[j * k1]);
+      v[k1] = cmul(v[k1], make_float2(w.x, -w.y));
+    }
+    C* yp = yb + p * N1 * N2P;
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) yp[k1 * N2P + j] = v[k1];
+  }
+  __syncthreads();
+  // I2: physical velocities
+  for (int it = threadIdx.x; it < NPI * N1; it += NT) {
+    const int p = it / N1, i = it % N1;
+    C w[N2];
+    const C* yp = yb + p * N1 * N2P + i * N2P;
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) w[n2] = yp[n2];
+    DFT<N2, true, C>::run(w);
+    float* oa;
+    float* ob;
+    if (p < TR) { oa = uph + (0 * TR + p) * N; ob = uph + (1 * TR + p) * N; }
+    else { const int q = p - TR; oa = uph + (2 * TR + 2 * q) * N; ob = uph + (2 * TR + 2 * q + 1) * N; }
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) { oa[i + N1 * k2] = w[k2].x; ob[i + N1 * k2] = w[k2].y; }
+  }
+  __syncthreads();
+  const float sc = float(a.scale);
+  const int K1o = a.K1out;
+  const long long ldo = a.ldo > 0 ? a.ldo : K1o;
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    // F1: products of the half's rows, forward step 1 (pencil p: row half*TH + p % TH, kind p / TH)
+    for (int it = threadIdx.x; it < NPF * N2; it += NT) {
+      const int p = it / N2, j = it % N2;
+      const int r = half * TH + p % TH, kind = p / TH;
+      const float* u1 = uph + (0 * TR + r) * N;
+      const float* u2 = uph + (1 * TR + r) * N;
+      const float* u3 = uph + (2 * TR + r) * N;
+      C v[N1];
+#pragma unroll
+      for (int n1 = 0; n1 < N1; ++n1) {
+        const int x = N2 * n1 + j;
+        const float a1 = u1[x], a2 = u2[x], a3 = u3[x];
+        v[n1] = kind == 0 ? make_float2(a1 * a1 * sc, a2 * a2 * sc)
+              : kind == 1 ? make_float2(a3 * a3 * sc, a1 * a2 * sc)
+                          : make_float2(a2 * a3 * sc, a3 * a1 * sc);
+      }
+      DFT<N1, false, C>::run(v);
+#pragma unroll
+      for (int k1 = 1; k1 < N1; ++k1) v[k1] = cmul(v[k1], __ldg(&tw[j * k1]));
+      C* yp = yb + p * N1 * N2P;
+#pragma unroll
+      for (int k1 = 0; k1 < N1; ++k1) yp[k1 * N2P + j] = v[k1];
+    }
+    __syncthreads();
+    // F2: forward step 2 into Z (the staged input rows are no longer needed)
+    for (int it = threadIdx.x; it < NPF * N1; it += NT) {
+      const int p = it / N1, i = it % N1;
+      C w[N2];
+      const C* yp = yb + p * N1 * N2P + i * N2P;
+#pragma unroll
+      for (int n2 = 0; n2 < N2; ++n2) w[n2] = yp[n2];
+      DFT<N2, false, C>::run(w);
+      C* zp = zb + p * ZS;
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2) {
+        const int k = i + N1 * k2;
+        if (k <= ko) zp[k] = w[k2];
+        else if (k >= N - ko) zp[ko + (N - k)] = w[k2];
+      }
+    }
+    __syncthreads();
+    // S: split and store the half's product rows
+    for (int it = threadIdx.x; it < TH * K1o; it += NT) {
+      const int rr = it / K1o, kx = it % K1o;
+      const long long row = row0 + half * TH + rr;
+      if (row >= a.nrows) continue;
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        const C* zp = zb + (b * TH + rr) * ZS;
+        const C z = zp[kx], zc = zp[kx == 0 ? 0 : ko + kx];
+        static_cast<C*>(a.out[2 * b])[row * ldo + kx] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
+        static_cast<C*>(a.out[2 * b + 1])[row * ldo + kx] = make_float2(0.5f * (z.y + zc.y), 0.5f * (zc.x - z.x));
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// r2c: two-level register FFT per pencil, a pencil being one row of two
+// components packed as a + i b
 template <int N> struct XPF;
-template <> struct XPF<810> { static constexpr int TP = 8; };
-template <> struct XPF<256> { static constexpr int TP = 16; };
 template <> struct XPF<128> { static constexpr int TP = 32; };
 template <> struct XPF<64> { static constexpr int TP = 32; };
 
@@ -850,97 +666,6 @@ template <int N> struct XPFCfg {
   static constexpr size_t SMEM = RIN + YB;
 };
 
-// Hermitian extension of one real row's half spectrum (K1 modes), the imaginary
-// parts of the mean and of the Nyquist mode dropped (a real row's c2r ignores them)
-template <int N> __device__ __forceinline__ float2 hext3(const float2* row, int K1, int f) {
-  const int kmax = K1 - 1;
-  if (f == 0) return make_float2(row[0].x, 0.f);
-  if (f <= kmax) {
-    float2 v = row[f];
-    if (2 * f == N) v.y = 0.f;
-    return v;
-  }
-  if (f >= N - kmax) { const float2 v = row[N - f]; return make_float2(v.x, -v.y); }
-  return make_float2(0.f, 0.f);
-}
-
-template <int N>
-__global__ void __launch_bounds__(XPFCfg<N>::NT) k_xc2r_fast(const XPlainArgs a, const float2* __restrict__ tw) {
-  using Cfg = XPFCfg<N>;
-  constexpr int N1 = Cfg::N1, N2 = Cfg::N2, N2P = Cfg::N2P, TP = Cfg::TP, NT = Cfg::NT, KMAX = Cfg::KMAX;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* rin = reinterpret_cast<float2*>(smem_raw);              // [TP][2][KMAX]
-  float2* yb = reinterpret_cast<float2*>(smem_raw + Cfg::RIN);    // [TP][N1][N2P]
-  // pencil, row and element indices stay 32-bit (at most 810^2 rows x 406
-  // modes per component); one warp stages one row, so no per-element division
-  const int npair = (a.ncomp + 1) / 2, K1 = a.K1;
-  const int npen = int(a.nrows) * npair, pen0 = blockIdx.x * TP;
-  // both loops have compile-time trip counts and are unrolled, so each thread
-  // issues all of its loads before the first store (a rolled loop waited out
-  // one global-load latency per element)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  static_assert((2 * TP) % (NT / 32) == 0, "whole rows per warp");
-#pragma unroll
-  for (int i = 0; i < 2 * TP / (NT / 32); ++i) {
-    const int s = warp + i * (NT / 32);
-    const int pen = pen0 + (s >> 1);
-    const float2* src = nullptr;
-    if (pen < npen) {
-      const int row = pen / npair, q = 2 * (pen - row * npair) + (s & 1);
-      if (q < a.ncomp) src = static_cast<const float2*>(a.in[q]) + row * K1;
-    }
-    float2* dst = rin + s * KMAX;
-#pragma unroll
-    for (int u = 0; u < (KMAX + 31) / 32; ++u) {
-      const int kx = lane + 32 * u;
-      if (kx < K1) dst[kx] = src ? __ldg(src + kx) : make_float2(0.f, 0.f);
-    }
-  }
-  __syncthreads();
-  for (int it = threadIdx.x; it < TP * N2; it += NT) {
-    const int p = it / N2, j = it - p * N2;
-    const float2* ra = rin + (p * 2) * KMAX;
-    const float2* rb = ra + KMAX;
-    float2 v[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-      const int f = N2 * n1 + j;
-      const float2 x = hext3<N>(ra, K1, f), y = hext3<N>(rb, K1, f);
-      v[n1] = make_float2(x.x - y.y, x.y + y.x);
-    }
-    DFT<N1, true, float2>::run(v);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1) {
-      const float2 w = __ldg(&tw[j * k1]);
-      v[k1] = cmul(v[k1], make_float2(w.x, -w.y));
-    }
-    float2* yp = yb + p * N1 * N2P;
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) yp[k1 * N2P + j] = v[k1];
-  }
-  __syncthreads();
-  const float sc = float(a.scale);
-  for (int it = threadIdx.x; it < TP * N1; it += NT) {
-    const int p = it / N1, i = it - p * N1;
-    const int pen = pen0 + p;
-    if (pen >= npen) continue;
-    float2 w[N2];
-    const float2* yp = yb + p * N1 * N2P + i * N2P;
-#pragma unroll
-    for (int n2 = 0; n2 < N2; ++n2) w[n2] = yp[n2];
-    DFT<N2, true, float2>::run(w);
-    const int row = pen / npair;
-    const int pr = pen - row * npair;
-    float* oa = static_cast<float*>(a.out[2 * pr]) + row * N + i;
-    float* ob = 2 * pr + 1 < a.ncomp ? static_cast<float*>(a.out[2 * pr + 1]) + row * N + i : nullptr;
-#pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) {
-      oa[N1 * k2] = w[k2].x * sc;
-      if (ob) ob[N1 * k2] = w[k2].y * sc;
-    }
-  }
-}
-
 template <int N>
 __global__ void __launch_bounds__(XPFCfg<N>::NT) k_xr2c_fast(const XPlainArgs a, const float2* __restrict__ tw) {
   using Cfg = XPFCfg<N>;
@@ -949,7 +674,7 @@ __global__ void __launch_bounds__(XPFCfg<N>::NT) k_xr2c_fast(const XPlainArgs a,
   float2* zb = reinterpret_cast<float2*>(smem_raw);               // [TP][2 KMAX]: kept outputs
   float2* yb = reinterpret_cast<float2*>(smem_raw + Cfg::RIN);    // [TP][N1][N2P]
   const int npair = (a.ncomp + 1) / 2, K1 = a.K1, ko = K1 - 1;
-  const int npen = int(a.nrows) * npair, pen0 = blockIdx.x * TP;  // 32-bit, as in k_xc2r_fast
+  const int npen = int(a.nrows) * npair, pen0 = blockIdx.x * TP;
   const float sc = float(a.scale);
   for (int it = threadIdx.x; it < TP * N2; it += NT) {
     const int p = it / N2, j = it - p * N2;
@@ -1012,74 +737,7 @@ __global__ void __launch_bounds__(XPFCfg<N>::NT) k_xr2c_fast(const XPlainArgs a,
   }
 }
 
-// ---------------------------------------------------------------------------
-// dispatch
-// ---------------------------------------------------------------------------
-template <typename F> static void set_smem2(F* f, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-}
-
-// Column-sweep variants the autotuner chooses from, per N: (tile width T,
-// split S).  Variant 0 is the default; launches with derivative outputs always
-// use variant 0.
-template <int N> struct ColVariants;
-template <> struct ColVariants<810> {
-  static constexpr int count = 4;
-  static constexpr int T[4] = {8, 8, 4, 16}, S[4] = {0, 1, 0, 0};
-};
-static_assert(ColVariants<810>::count == kColTmaVariant, "the TMA-fed sweep follows the k_col2 variants");
-template <> struct ColVariants<256> {
-  static constexpr int count = 2;
-  static constexpr int T[2] = {16, 8}, S[2] = {0, 0};
-};
-template <> struct ColVariants<128> {
-  static constexpr int count = 3;
-  static constexpr int T[3] = {16, 8, 16}, S[3] = {0, 0, 1};
-};
-template <> struct ColVariants<64> {
-  static constexpr int count = 2;
-  static constexpr int T[2] = {16, 8}, S[2] = {0, 0};
-};
-
-template <int N, int T, int S> static void init_col2_variant() {
-  using Cfg = Col2Cfg<N, T, S>;
-  set_smem2(k_col2<N, T, true, false, false, S>, Cfg::SMEM);
-  set_smem2(k_col2<N, T, true, false, true, S>, Cfg::SMEM);
-  set_smem2(k_col2<N, T, false, false, false, S>, Cfg::SMEM);
-  set_smem2(k_col2<N, T, false, false, true, S>, Cfg::SMEM);
-}
-
-template <int N, int V = 0> static void init_col2_variants() {
-  if constexpr (V < ColVariants<N>::count) {
-    init_col2_variant<N, ColVariants<N>::T[V], ColVariants<N>::S[V]>();
-    init_col2_variants<N, V + 1>();
-  }
-}
-
-template <int N> static void init_xplain();
-
-template <int N> static void init_fast_n() {
-  constexpr int T = ColVariants<N>::T[0];
-  set_smem2(k_col2<N, T, true, true, false>, Col2Cfg<N, T>::SMEM);
-  set_smem2(k_col2<N, T, true, true, true>, Col2Cfg<N, T>::SMEM);
-  init_col2_variants<N>();
-  set_smem2(k_xsweep2<N, 2>, X2Cfg<N, 2>::SMEM);
-  set_smem2(k_xsweep2<N, 3>, X2Cfg<N, 3>::SMEM);
-  set_smem2(k_xsweep3<N>, X3Cfg<N>::SMEM);
-  if (N == 810) set_smem2(k_xsweep4<true>, X4Cfg::SMEM), set_smem2(k_xsweep4<false>, X4Cfg::SMEM);
-  init_xplain<N>();
-}
-
-bool fast_supported(int N) { return N == 810 || N == 256 || N == 128 || N == 64; }
-
-template <int N> static void init_xplain() {
-  set_smem2(k_xc2r_fast<N>, XPFCfg<N>::SMEM);
-  set_smem2(k_xr2c_fast<N>, XPFCfg<N>::SMEM);
-}
-
-// ---------------------------------------------------------------------------
-// x c2r for N = 64 and 128 with one warp per packed row pair, in registers
-// ---------------------------------------------------------------------------
+// c2r, one warp per pencil in registers:
 // Z[f] = X_a[f] + i X_b[f] (the Hermitian extensions of two real rows' half
 // spectra); lane l holds Z[l + 32 q], q < Q = N / 32.  A radix-Q inverse DFT
 // over q and the twiddles exp(+2 pi i l k1 / N) in registers, then for each
@@ -1148,30 +806,63 @@ __global__ void __launch_bounds__(256) k_xc2r_warp(const XPlainArgs a, const flo
   }
 }
 
-template <int N> static void xplain_n(bool inv, const XPlainArgs& a, const void* tw, cudaStream_t st) {
-  using Cfg = XPFCfg<N>;
-  const long long npen = a.nrows * ((a.ncomp + 1) / 2);
-  const unsigned nb = unsigned((npen + Cfg::TP - 1) / Cfg::TP);
-  const float2* t2 = static_cast<const float2*>(tw);
-  if (inv && (N == 64 || N == 128)) {
-    k_xc2r_warp<N == 64 ? 64 : 128><<<unsigned((npen + 7) / 8), 256, 0, st>>>(a, t2);
-    return;
-  }
-  if (inv) k_xc2r_fast<N><<<nb, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
-  else k_xr2c_fast<N><<<nb, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
+// ---------------------------------------------------------------------------
+// dispatch
+// ---------------------------------------------------------------------------
+template <typename F> static void set_smem2(F* f, size_t bytes) {
+  if (bytes > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
 }
 
-bool launch_xplain_fast(int N, bool inv, const XPlainArgs& a, const void* tw, cudaStream_t st) {
-  if (a.K1 > N / 2 + 1 || a.K1 < 1) return false;
-  if (a.nrows * N >= (1ll << 31)) return false;  // the kernels index rows and elements in 32 bits
-  switch (N) {
-    case 810: xplain_n<810>(inv, a, tw, st); return true;
-    case 256: xplain_n<256>(inv, a, tw, st); return true;
-    case 128: xplain_n<128>(inv, a, tw, st); return true;
-    case 64: xplain_n<64>(inv, a, tw, st); return true;
-    default: return false;
+// Column-sweep variants the autotuner chooses from, per N: (tile width T,
+// split S).  Variant 0 is the default; launches with derivative outputs always
+// use variant 0.
+template <int N> struct ColVariants;
+template <> struct ColVariants<810> {
+  static constexpr int count = 4;
+  static constexpr int T[4] = {8, 8, 4, 16}, S[4] = {0, 1, 0, 0};
+};
+static_assert(ColVariants<810>::count == kColTmaVariant, "the TMA-fed sweep follows the k_col2 variants");
+template <> struct ColVariants<256> {
+  static constexpr int count = 2;
+  static constexpr int T[2] = {16, 8}, S[2] = {0, 0};
+};
+template <> struct ColVariants<128> {
+  static constexpr int count = 3;
+  static constexpr int T[3] = {16, 8, 16}, S[3] = {0, 0, 1};
+};
+template <> struct ColVariants<64> {
+  static constexpr int count = 2;
+  static constexpr int T[2] = {16, 8}, S[2] = {0, 0};
+};
+
+template <int N, int T, int S> static void init_col2_variant() {
+  using Cfg = Col2Cfg<N, T, S>;
+  set_smem2(k_col2<N, T, true, false, false, S>, Cfg::SMEM);
+  set_smem2(k_col2<N, T, true, false, true, S>, Cfg::SMEM);
+  set_smem2(k_col2<N, T, false, false, false, S>, Cfg::SMEM);
+  set_smem2(k_col2<N, T, false, false, true, S>, Cfg::SMEM);
+}
+
+template <int N, int V = 0> static void init_col2_variants() {
+  if constexpr (V < ColVariants<N>::count) {
+    init_col2_variant<N, ColVariants<N>::T[V], ColVariants<N>::S[V]>();
+    init_col2_variants<N, V + 1>();
   }
 }
+
+template <int N> static void init_fast_n() {
+  constexpr int T = ColVariants<N>::T[0];
+  set_smem2(k_col2<N, T, true, true, false>, Col2Cfg<N, T>::SMEM);
+  set_smem2(k_col2<N, T, true, true, true>, Col2Cfg<N, T>::SMEM);
+  init_col2_variants<N>();
+  if constexpr (N == 64 || N == 128) {
+    set_smem2(k_xsweep3<N>, X3Cfg<N>::SMEM);
+    set_smem2(k_xr2c_fast<N>, XPFCfg<N>::SMEM);
+  }
+  if (N == 810) set_smem2(k_xsweep4<true>, X4Cfg::SMEM), set_smem2(k_xsweep4<false>, X4Cfg::SMEM);
+}
+
+bool fast_supported(int N) { return N == 810 || N == 256 || N == 128 || N == 64; }
 
 bool init_fast(int N) {
   switch (N) {
@@ -1245,48 +936,58 @@ int col2_variants(int N) {
   }
 }
 
-// x-sweep variants (3D): at 810, 0 = the scalar three-level sweep (default:
-// the fastest measured), 1 = the paired-row f32x2 sweep at five CTAs per SM,
-// 2 = the same at four CTAs per SM (registers for its twiddles), 3 = the
-// two-level sweep of four rows per CTA; elsewhere 0 = the two-level four-row-
-// group sweep, 1 = the plain two-level sweep.
-template <int N> static void x2_n(const XArgs& a, const void* tw, cudaStream_t st) {
-  const float2* t2 = static_cast<const float2*>(tw);
-  const unsigned nb = unsigned((a.nrows + X2Rows<N>::TR - 1) / X2Rows<N>::TR);
-  const unsigned nb3 = unsigned((a.nrows + X3Rows<N>::TR - 1) / X3Rows<N>::TR);
-  if (a.D == 2) {
-    k_xsweep2<N, 2><<<nb, X2Cfg<N, 2>::NT, X2Cfg<N, 2>::SMEM, st>>>(a, t2);
-  } else if (N == 810) {
-    if (a.variant == 1 || a.variant == 2) {
-      launch_xpair810(a, t2 + 810, a.variant == 2 ? 4 : 5, st);
-    } else if (a.variant == 3) {
-      k_xsweep3<N><<<nb3, X3Cfg<N>::NT, X3Cfg<N>::SMEM, st>>>(a, t2);
-    } else {
-      const unsigned nb4 = unsigned((a.nrows + 1) / 2);
-      if (a.K1in == 271 && a.K1out == 271) k_xsweep4<true><<<nb4, X4Cfg::NT, X4Cfg::SMEM, st>>>(a, t2);
-      else k_xsweep4<false><<<nb4, X4Cfg::NT, X4Cfg::SMEM, st>>>(a, t2);
-    }
-  } else if (a.variant == 1) {
-    k_xsweep2<N, 3><<<nb, X2Cfg<N, 3>::NT, X2Cfg<N, 3>::SMEM, st>>>(a, t2);
-  } else {
-    k_xsweep3<N><<<nb3, X3Cfg<N>::NT, X3Cfg<N>::SMEM, st>>>(a, t2);
-  }
-}
-
+// x-sweep variants of the 3D product sweep: at 810, 0 = the scalar three-level
+// sweep (the fastest measured: 904 us for 102 500 rows), 1 = the paired-row
+// f32x2 sweep at five CTAs per SM, 2 = the same at four CTAs per SM (registers
+// for its twiddles), 3 = the warp-per-row-pair sweep of the other sizes (1096
+// us: a warp of 30 x 27 points holds too many registers to keep the issue slots
+// busy).  At 64 and 128, 0 = the warp-per-row-pair sweep and 1 = the CTA-wide
+// sweep above; 256 has the first only and takes 1 for it too.
 int xsweep_variants(int N, int D) {
   if (D != 3 || !fast_supported(N)) return 1;
   return N == 810 ? 4 : 2;
 }
 
-bool launch_xsweep2(int N, const XArgs& a, const void* tw, cudaStream_t st) {
-  if (a.K1in > N / 3 + 1 || a.K1out > a.K1in) return false;
-  switch (N) {
-    case 810: x2_n<810>(a, tw, st); return true;
-    case 256: x2_n<256>(a, tw, st); return true;
-    case 128: x2_n<128>(a, tw, st); return true;
-    case 64: x2_n<64>(a, tw, st); return true;
-    default: return false;
+template <int N> static void xsweep3_n(const XArgs& a, const float2* t2, cudaStream_t st) {
+  const unsigned nb = unsigned((a.nrows + X3Rows<N>::TR - 1) / X3Rows<N>::TR);
+  k_xsweep3<N><<<nb, X3Cfg<N>::NT, X3Cfg<N>::SMEM, st>>>(a, t2);
+}
+
+bool launch_xsweep3(int N, const XArgs& a, const void* tw, cudaStream_t st) {
+  if (a.D != 3 || a.variant != 1) return false;
+  const float2* t2 = static_cast<const float2*>(tw);
+  if (N == 64) xsweep3_n<64>(a, t2, st);
+  else if (N == 128) xsweep3_n<128>(a, t2, st);
+  else return false;
+  return true;
+}
+
+template <int N> static void xplain_n(bool inv, const XPlainArgs& a, const float2* t2, cudaStream_t st) {
+  using Cfg = XPFCfg<N>;
+  const long long npen = a.nrows * ((a.ncomp + 1) / 2);
+  if (inv) k_xc2r_warp<N><<<unsigned((npen + 7) / 8), 256, 0, st>>>(a, t2);
+  else k_xr2c_fast<N><<<unsigned((npen + Cfg::TP - 1) / Cfg::TP), Cfg::NT, Cfg::SMEM, st>>>(a, t2);
+}
+
+bool launch_xplain_pinned(int N, bool inv, const XPlainArgs& a, const void* tw, cudaStream_t st) {
+  const float2* t2 = static_cast<const float2*>(tw);
+  if (N == 64) xplain_n<64>(inv, a, t2, st);
+  else if (N == 128) xplain_n<128>(inv, a, t2, st);
+  else return false;
+  return true;
+}
+
+bool launch_xsweep810(const XArgs& a, const void* tw, cudaStream_t st) {
+  if (a.D != 3 || a.variant == 3) return false;
+  const float2* t2 = static_cast<const float2*>(tw);
+  if (a.variant == 1 || a.variant == 2) {
+    launch_xpair810(a, t2 + 810, a.variant == 2 ? 4 : 5, st);
+    return true;
   }
+  const unsigned nb4 = unsigned((a.nrows + 1) / 2);
+  if (a.K1in == 271 && a.K1out == 271) k_xsweep4<true><<<nb4, X4Cfg::NT, X4Cfg::SMEM, st>>>(a, t2);
+  else k_xsweep4<false><<<nb4, X4Cfg::NT, X4Cfg::SMEM, st>>>(a, t2);
+  return true;
 }
 
 }  // namespace sc

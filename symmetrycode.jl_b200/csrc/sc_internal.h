@@ -59,6 +59,7 @@ struct XPlainArgs {
   int K1;          // spectral row extent (kx = 0..K1-1)
   long long nrows;
   double scale;    // applied to the output
+  bool pinned;     // FP32 n = 64, 128: the kernels of the one-pass BF16 network (launch_xplain_pinned)
 };
 
 // Pointwise spectral epilogue over the compact 2/3 cube (see k_epilogue).
@@ -114,7 +115,7 @@ template <typename R> bool launch_x_c2r(int N, const XPlainArgs& a, const void* 
 template <typename R> bool launch_x_r2c(int N, const XPlainArgs& a, const void* tw, cudaStream_t st);
 template <typename R> void launch_epilogue(const EpiArgs& a, cudaStream_t st);
 template <typename R> void launch_filter(const FilterArgs& a, cudaStream_t st);
-// max |u| over the physical points of D rows-of-spectra (x inverse fused with the reduction)
+// max |u|^2 over the physical points of D rows-of-spectra (x inverse fused with the reduction)
 template <typename R> bool launch_x_vmax(int N, const XPlainArgs& a, const void* tw, unsigned long long* out,
                                          cudaStream_t st);
 // shells 1..2 on the compact state held in a.dst: mode 0 measures into eref[0..1], mode 1 rescales
@@ -136,7 +137,11 @@ bool fft_size_supported(int n);
 bool fast_supported(int N);
 bool init_fast(int N);
 bool launch_col2(int N, bool inv, const ColArgs& a, const void* tw, cudaStream_t st);
-bool launch_xsweep2(int N, const XArgs& a, const void* tw, cudaStream_t st);
+// the x sweeps around the one-pass BF16 closure network, N = 64 and 128 (sc_fast.cu)
+bool launch_xsweep3(int N, const XArgs& a, const void* tw, cudaStream_t st);
+bool launch_xplain_pinned(int N, bool inv, const XPlainArgs& a, const void* tw, cudaStream_t st);
+// 3D product sweep of N = 810 (false: the variant is the general sweep of sc_xrow.h)
+bool launch_xsweep810(const XArgs& a, const void* tw, cudaStream_t st);
 // randomfield on the device (sc_random.cu): counter-based N(0, 1/2) draws into
 // the FP64 compact work arrays w, then symmetrize!, project!, twothirds! and
 // the per-shell rescale to target[s] (eshell: smax + 1 zeroed doubles) into
@@ -145,8 +150,6 @@ void launch_random_draws(void* const* w, int D, int K1, int kc, unsigned long lo
 template <typename R>
 void launch_random_finish(void* const* w, void* const* out, int D, int n, int K1, int kc, double* eshell,
                           const double* target, cudaStream_t st);
-// FP32 plain c2r (inv) / r2c along x for the fast sizes (sc_fast.cu); false when not applicable
-bool launch_xplain_fast(int N, bool inv, const XPlainArgs& a, const void* tw, cudaStream_t st);
 // number of autotuner variants of the FP32 column sweeps / 3D x sweep of size N
 int col2_variants(int N);
 // TMA-fed persistent column sweeps for N = 810 (sc_coltma.cu): column-sweep
@@ -164,10 +167,14 @@ size_t xpair810_twiddle_bytes();
 void xpair810_twiddles(const float2* tw, float* out8);
 bool init_xpair810();
 void launch_xpair810(const XArgs& a, const void* twp_table, int minb, cudaStream_t st);
-// bytes of a plan's twiddle buffer: the plain table plus, for FP32 n = 810, the pair table
-inline size_t twiddle_buffer_bytes(int n, size_t esz) {
+// A plan's twiddle buffer: the plain table exp(-2 pi i j / n); for FP32 n = 810
+// the pair table; then the x sweep's two tables in the order its lanes read
+// them, exp(-2 pi i a b / n) at [a][b] for a < N1, b < N2 and for a < N2, b < N1
+// (sc_sweep_sizes.h).
+inline size_t twiddle_x_offset(int n, size_t esz) {
   return (size_t)n * esz + (esz == 8 && n == 810 ? xpair810_twiddle_bytes() : 0);
 }
+inline size_t twiddle_buffer_bytes(int n, size_t esz) { return twiddle_x_offset(n, esz) + 2 * (size_t)n * esz; }
 template <typename R> bool init_kernels(int N);
 template <typename R> void launch_twothirds_full(const PackArgs& a, cudaStream_t st);  // in place on a.dst
 template <typename R> void launch_project_full(const PackArgs& a, double kfac, cudaStream_t st);

@@ -15,6 +15,7 @@
 // zero modes `twothirds!` (src/solver.jl:371-389) would mask are never read.
 #include "sc_fft.cuh"
 #include "sc_internal.h"
+#include "sc_xrow.h"
 
 #include <cstdlib>
 #include <cstring>
@@ -624,7 +625,7 @@ __global__ void k_spectral_energy(const PackArgs a, int K1, int K2, int compact,
 // ---------------------------------------------------------------------------
 // CFL velocity maximum, shell clamp, spectrum
 // ---------------------------------------------------------------------------
-// max over physical points of |u| from D spectral x-rows (propose_timestep,
+// max over physical points of |u|^2 from D spectral x-rows (propose_timestep,
 // src/solver.jl:931-947); the rows hold the y/z-inverse transforms of P u.
 // Result as float bits (non-negative floats order like their bit patterns).
 template <typename R, int N>
@@ -654,7 +655,7 @@ k_x_vmax(const XPlainArgs a, const typename V2<R>::T* __restrict__ tw, unsigned 
     const int t = idx / N;
     if (row0 + t >= a.nrows) continue;
     const C z1 = s[idx], z2 = s[TR * N + idx];
-    const double v = sqrt(double(z1.x) * z1.x + double(z1.y) * z1.y + double(z2.x) * z2.x);
+    const double v = double(z1.x) * z1.x + double(z1.y) * z1.y + double(z2.x) * z2.x;
     m = v > m ? v : m;
   }
 #pragma unroll
@@ -750,6 +751,10 @@ __global__ void k_spectrum(const PackArgs a, int nshell, double* s) {
   X(90) X(96) X(120) X(128) X(160) X(180) X(192) X(240) X(256) X(270) X(320) X(360) X(384) X(512) X(540) \
   X(640) X(720) X(768) X(810) X(1024)
 
+// sizes whose x transforms run on the shared-memory engine; the others are those
+// of sc_sweep_sizes.h
+#define SC_SIZES_SMALL(X) X(4) X(6) X(8) X(10) X(12) X(16) X(18) X(20) X(24) X(30)
+
 bool fft_size_supported(int n) {
   switch (n) {
 #define SC_CASE(N) case N: return true;
@@ -806,10 +811,12 @@ static bool xr2c_n(const XPlainArgs& a, const void* tw, cudaStream_t st) {
 template <typename R, int N> static bool init_n() {
   set_smem(k_col_inv<R, N>, ColCfg<R, N>::SMEM);
   set_smem(k_col_fwd<R, N>, ColCfg<R, N>::SMEM);
-  set_smem(k_xsweep_ns<R, N, 2>, XCfg<R, N>::SMEM);
-  set_smem(k_xsweep_ns<R, N, 3>, XCfg<R, N>::SMEM);
-  set_smem(k_x_c2r<R, N>, XPCfg<R, N>::SMEM);
-  set_smem(k_x_r2c<R, N>, XPCfg<R, N>::SMEM);
+  if constexpr (N < 32) {
+    set_smem(k_xsweep_ns<R, N, 2>, XCfg<R, N>::SMEM);
+    set_smem(k_xsweep_ns<R, N, 3>, XCfg<R, N>::SMEM);
+    set_smem(k_x_c2r<R, N>, XPCfg<R, N>::SMEM);
+    set_smem(k_x_r2c<R, N>, XPCfg<R, N>::SMEM);
+  }
   return cudaGetLastError() == cudaSuccess;
 }
 
@@ -817,6 +824,7 @@ template <typename R, int N> static bool init_n() {
 // process and device, before any launch or stream capture).
 template <typename R> bool init_kernels(int N) {
   if (sizeof(R) == 4 && fast_supported(N) && !init_fast(N)) return false;
+  if (!xrow_init<R>(N)) return false;
   switch (N) {
 #define SC_CASE(NN) case NN: return init_n<R, NN>();
     SC_SIZES(SC_CASE)
@@ -848,28 +856,32 @@ template <typename R> bool launch_col_fwd(int N, const ColArgs& a, const void* t
   }
 }
 template <typename R> bool launch_xsweep_ns(int N, const XArgs& a, const void* tw, cudaStream_t st) {
-  if (use_fast<R>(N) && launch_xsweep2(N, a, tw, st)) return true;
+  if (sizeof(R) == 4 && launch_xsweep3(N, a, tw, st)) return true;
+  if (sizeof(R) == 4 && N == 810 && launch_xsweep810(a, tw, st)) return true;
+  if (xrow_ns<R>(N, a, tw, st)) return true;
   switch (N) {
 #define SC_CASE(NN) case NN: return xsweep_n<R, NN>(a, tw, st);
-    SC_SIZES(SC_CASE)
+    SC_SIZES_SMALL(SC_CASE)
 #undef SC_CASE
     default: return false;
   }
 }
 template <typename R> bool launch_x_c2r(int N, const XPlainArgs& a, const void* tw, cudaStream_t st) {
-  if (use_fast<R>(N) && launch_xplain_fast(N, true, a, tw, st)) return true;
+  if (sizeof(R) == 4 && a.pinned && launch_xplain_pinned(N, true, a, tw, st)) return true;
+  if (xrow_c2r<R>(N, a, tw, st)) return true;
   switch (N) {
 #define SC_CASE(NN) case NN: return xc2r_n<R, NN>(a, tw, st);
-    SC_SIZES(SC_CASE)
+    SC_SIZES_SMALL(SC_CASE)
 #undef SC_CASE
     default: return false;
   }
 }
 template <typename R> bool launch_x_r2c(int N, const XPlainArgs& a, const void* tw, cudaStream_t st) {
-  if (use_fast<R>(N) && launch_xplain_fast(N, false, a, tw, st)) return true;
+  if (sizeof(R) == 4 && a.pinned && launch_xplain_pinned(N, false, a, tw, st)) return true;
+  if (xrow_r2c<R>(N, a, tw, st)) return true;
   switch (N) {
 #define SC_CASE(NN) case NN: return xr2c_n<R, NN>(a, tw, st);
-    SC_SIZES(SC_CASE)
+    SC_SIZES_SMALL(SC_CASE)
 #undef SC_CASE
     default: return false;
   }
@@ -893,9 +905,10 @@ template <typename R, int N> static bool xvmax_n(const XPlainArgs& a, const void
 
 template <typename R> bool launch_x_vmax(int N, const XPlainArgs& a, const void* tw, unsigned long long* out,
                                          cudaStream_t st) {
+  if (xrow_vmax<R>(N, a, tw, out, st)) return true;
   switch (N) {
 #define SC_CASE(NN) case NN: return xvmax_n<R, NN>(a, tw, out, st);
-    SC_SIZES(SC_CASE)
+    SC_SIZES_SMALL(SC_CASE)
 #undef SC_CASE
     default: return false;
   }

@@ -1,0 +1,52 @@
+// Sizes of the two-level register sweeps and how each length is split.
+//
+// X(N, xf1, xf2, xd1, xd2, c1, c2): N = xf1 * xf2 splits the x rows in FP32
+// (xf1 lanes of a warp hold xf2 points each between the inverse and the
+// forward transform), N = xd1 * xd2 in FP64, N = c1 * c2 the column sweeps
+// (radix c1 first).  Chosen so that xf1 fills the 32 lanes (a warp takes
+// 32 / xf1 row pairs) and 3 * (32 / xf1) * xf2, the work items of the other
+// radix pass, fills whole rounds of 32; the points per lane are what the
+// registers hold (about 6 values per point), so FP64 takes fewer of them.
+// Sizes below 32 keep the shared-memory engine of sc_kernels.cu.
+#pragma once
+
+#define SC_SWEEP_SIZES_A(X) \
+  X(32, 8, 4, 8, 4, 8, 4) X(36, 6, 6, 6, 6, 6, 6) X(40, 8, 5, 8, 5, 8, 5) X(48, 6, 8, 6, 8, 8, 6) \
+  X(60, 6, 10, 6, 10, 10, 6) X(64, 8, 8, 8, 8, 8, 8) X(72, 8, 9, 8, 9, 9, 8) X(80, 8, 10, 8, 10, 10, 8) \
+  X(90, 10, 9, 10, 9, 10, 9) X(96, 8, 12, 8, 12, 12, 8)
+#define SC_SWEEP_SIZES_B(X) \
+  X(120, 8, 15, 15, 8, 12, 10) X(128, 8, 16, 16, 8, 16, 8) X(160, 16, 10, 16, 10, 16, 10) \
+  X(180, 15, 12, 15, 12, 15, 12) X(192, 16, 12, 16, 12, 16, 12) X(240, 16, 15, 16, 15, 16, 15) \
+  X(256, 16, 16, 16, 16, 16, 16)
+#define SC_SWEEP_SIZES_C(X) \
+  X(270, 30, 9, 30, 9, 18, 15) X(320, 32, 10, 32, 10, 20, 16) X(360, 15, 24, 30, 12, 20, 18) \
+  X(384, 32, 12, 32, 12, 24, 16) X(512, 32, 16, 32, 16, 32, 16)
+#define SC_SWEEP_SIZES_D(X) \
+  X(540, 30, 18, 30, 18, 27, 20) X(640, 32, 20, 32, 20, 32, 20) X(720, 30, 24, 30, 24, 30, 24) \
+  X(768, 32, 24, 32, 24, 32, 24) X(810, 30, 27, 30, 27, 27, 30) X(1024, 32, 32, 32, 32, 32, 32)
+#define SC_SWEEP_SIZES(X) SC_SWEEP_SIZES_A(X) SC_SWEEP_SIZES_B(X) SC_SWEEP_SIZES_C(X) SC_SWEEP_SIZES_D(X)
+
+namespace sc {
+
+template <typename R, int N> struct XSplit;  // lanes N1, points per lane N2
+template <int N> struct CSplit;              // first radix N1, second radix N2
+#define SC_SPLIT(N, A1, A2, B1, B2, C1, C2)                                                             \
+  template <> struct XSplit<float, N> { static constexpr int N1 = A1, N2 = A2; };                       \
+  template <> struct XSplit<double, N> { static constexpr int N1 = B1, N2 = B2; };                      \
+  template <> struct CSplit<N> { static constexpr int N1 = C1, N2 = C2; };                              \
+  static_assert(A1 * A2 == N && B1 * B2 == N && C1 * C2 == N && A1 <= 32 && B1 <= 32, "split of N");
+SC_SWEEP_SIZES(SC_SPLIT)
+#undef SC_SPLIT
+
+// sizes with two-level sweeps; xn1 / xn2: the x split (for the host's twiddle tables)
+inline bool sweep_size(int n, bool f32, int* xn1 = nullptr, int* xn2 = nullptr) {
+  switch (n) {
+#define SC_CASE(N, A1, A2, B1, B2, C1, C2) \
+  case N: if (xn1) { *xn1 = f32 ? A1 : B1; *xn2 = f32 ? A2 : B2; } return true;
+    SC_SWEEP_SIZES(SC_CASE)
+#undef SC_CASE
+    default: return false;
+  }
+}
+
+}  // namespace sc

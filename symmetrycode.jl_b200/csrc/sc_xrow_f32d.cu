@@ -1,0 +1,8 @@
+// x sweeps of one precision and group of sizes (one object each, so that they compile in parallel).
+#include "sc_xrow.cuh"
+
+namespace sc {
+#define SC_CASE(N, ...) template struct XRow<float, N>;
+SC_SWEEP_SIZES_D(SC_CASE)
+#undef SC_CASE
+}  // namespace sc

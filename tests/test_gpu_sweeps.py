@@ -1,0 +1,90 @@
+"""The warp-per-row-pair x sweeps at every size they have, against the oracles.
+
+Every size is 2^a 3^b 5^c with its own split into lanes and points per lane, so
+each has its own remainders: lanes left over in a warp, work items left over in
+a round, the block of modes that straddles the 2/3 cut.  2D grids run the 2D
+product sweep, the plain transforms in the full layout and the CFL maximum; 3D
+grids run the 3D product sweep on a sparse field that reaches the cube's faces
+and corners, against exact triad sums.
+
+Tolerances (as in test_gpu_solver.py): FP64 1e-12 relative L2; FP32 1e-5 for a
+right-hand side and 1e-6 for one transform (a length-N transform in FP32 is off
+by about 6e-8 sqrt(log2 N^D) <= 3e-7).
+"""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+import oracle as O
+import symcode as S
+from _util import rel_l2, to_dev, to_np
+from oracle import triad as T
+
+pytestmark = pytest.mark.gpu
+
+SIZES = (32, 36, 40, 48, 60, 64, 72, 80, 90, 96, 120, 128, 160, 180, 192, 240, 256, 270, 320, 360, 384, 512, 540, 640,
+         720, 768, 810, 1024)
+DTYPES = (torch.float32, torch.float64)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n", SIZES)
+def test_2d_sweeps_match_the_oracle(n, dtype):
+    g, go = S.Grid(2, n, dtype=dtype, device="cuda:0"), O.Grid(2, n, 2 * math.pi)
+    tol, ftol = (1e-12, 1e-12) if dtype == torch.float64 else (1e-5, 1e-6)
+    u = O.random_field(go, 3, kpeak=5.0)
+    du = S.convectiondiffusion_(S.vectorfield(g), [to_dev(c, g) for c in u], g, 1e-3)
+    ref = [O.twothirds(c, go) for c in O.convectiondiffusion(u, go, 1e-3)]
+    assert rel_l2([to_np(c) for c in du], ref) < tol
+    dt = S.propose_timestep([to_dev(c, g) for c in u], g, 1e-6)
+    assert abs(dt / O.propose_timestep(u, go, 1e-6) - 1) < ftol
+    x = np.random.default_rng(n).standard_normal(go.phys_shape)
+    xd = to_dev(x, g)
+    spec = S.to_spec_(S.scalarfield(g), xd, g)
+    assert rel_l2(to_np(spec), O.to_spec(to_np(xd), go)) < ftol
+    back = S.to_phys_(S.spacescalarfield(g), spec, g)
+    assert rel_l2(to_np(back), to_np(xd)) < ftol
+
+
+@pytest.mark.parametrize("n", (32, 48, 90, 128))
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_3d_transforms_match_pocketfft(n, dtype):
+    """One field in 3D: the last warp's pencils are partly empty."""
+    g, go = S.Grid(3, n, dtype=dtype, device="cuda:0"), O.Grid(3, n, 2 * math.pi)
+    tol = 1e-12 if dtype == torch.float64 else 1e-6
+    xd = to_dev(np.random.default_rng(n).standard_normal(go.phys_shape), g)
+    spec = S.to_spec_(S.scalarfield(g), xd, g)
+    assert rel_l2(to_np(spec), O.to_spec(to_np(xd), go)) < tol
+    assert rel_l2(to_np(S.to_phys_(S.spacescalarfield(g), spec, g)), to_np(xd)) < tol
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n", SIZES)
+def test_3d_product_sweep_matches_triad_sums(n, dtype):
+    if n == 1024 and dtype == torch.float64:
+        pytest.skip("the plan and its fields do not fit one GPU")
+    k = n // 3
+    edges = ((k, 0, 0), (0, k, 0), (0, 0, k), (k, k, k), (k, -k, 1), (1, 0, 0), (0, 1, -1))
+    kk, uu = T.random_sparse_field(n, 40, n, extra=edges)
+    kout, ref = T.convectiondiffusion(kk, uu, n, 1e-3)
+    g = S.Grid(3, n, dtype=dtype, device="cuda:0")
+    kf, uf = T.full_modes(kk, uu)
+    half = kf[:, 0] >= 0
+    at = tuple(torch.from_numpy(a).to(g.device) for a in T.to_rfft_index(kf[half], n))
+    u = S.vectorfield(g)
+    for c in range(3):
+        u[c][at] = torch.from_numpy(uf[half][:, c]).to(g.cdtype).to(g.device)
+    du = S.convectiondiffusion_(S.vectorfield(g), u, g, 1e-3)
+    ot = tuple(torch.from_numpy(a).to(g.device) for a in T.to_rfft_index(kout, n))
+    num = den = 0.0
+    for c in range(3):
+        r = torch.from_numpy(ref[:, c]).to(g.device)
+        num += float((du[c][ot].to(torch.complex128) - r).abs().square().sum())
+        den += float(r.abs().square().sum())
+        du[c][ot] = 0  # what is left must be zero, and counts as error
+        num += float(torch.linalg.vector_norm(du[c]).double() ** 2)
+    assert math.sqrt(num / den) < (1e-12 if dtype == torch.float64 else 1e-5)
+    g.close()
