@@ -308,7 +308,7 @@ bool colt_init() { return set_attr<8, 2>() && set_attr<16, 2>() && set_attr<8, 3
 // smaller times its extent).  Returns false otherwise (the caller launches
 // k_col2).
 bool launch_colt(int N, bool inv, const ColArgs& a, const void* tw, int which, cudaStream_t st) {
-  if (N != kN || a.ndrv > 0 || a.zero_origin || a.kpos != kKP || a.kneg != kKN) return false;
+  if (N != kN || a.zero_origin || a.kpos != kKP || a.kneg != kKN) return false;
   if (a.ncomp < 1 || a.ncomp > kMaxComp || a.K1 < 1 || a.ncols < 1 || !a.err) return false;
   if ((a.in_es & 1) || (a.in_cs & 1)) return false;
   for (int q = 0; q < a.ncomp; ++q)

@@ -1,144 +1,16 @@
-// Two-level register FFT sweeps for the FP32 solver sizes (sm_100a).
-//
-// A length-N transform is split N = N1 * N2 (810 = 27 * 30, 256 = 16 * 16,
-// 128 = 16 * 8, 64 = 8 * 8):
-//   step 1  thread (pencil, n2) gathers x[N2 n1 + n2], n1 = 0..N1-1, straight
-//           from global memory into registers, runs a radix-N1 DFT in
-//           registers, multiplies by exp(-+2 pi i n2 k1 / N) and writes one
-//           row of the shared exchange buffer;
-//   step 2  thread (pencil, k1) reads the N2 values of its column, runs a
-//           radix-N2 DFT in registers and stores X[k1 + N1 k2] straight to
-//           global memory (pruned to the retained modes on the forward side).
-// Each element crosses shared memory once (one store, one load) instead of
-// once per radix pass, and every thread keeps N1 independent global loads in
-// flight.  These kernels replace the Stockham-engine sweeps of sc_kernels.cu
-// for FP32 at the sizes of the DNS and LES configurations; the results are the
-// same transforms (tests compare both against the FP64 oracle).
+// FP32 kernels of the solver's own sizes (sm_100a): the column-sweep variants the
+// autotuner chooses from, the three-level x sweep of 810, and the x sweeps around
+// the one-pass BF16 closure network.
+#include "sc_col.cuh"
 #include "sc_fft.cuh"
 #include "sc_internal.h"
 
 namespace sc {
 
-// N = N1 * N2 of the two-level column sweeps; S = 1 is the transposed split,
-// one of the autotuner's candidates (the x sweeps use S = 0).
-template <int N, int S = 0> struct Split;
-template <> struct Split<810, 0> { static constexpr int N1 = 27, N2 = 30; };
-template <> struct Split<810, 1> { static constexpr int N1 = 30, N2 = 27; };
-template <> struct Split<256, 0> { static constexpr int N1 = 16, N2 = 16; };
-template <> struct Split<256, 1> { static constexpr int N1 = 16, N2 = 16; };
-template <> struct Split<128, 0> { static constexpr int N1 = 16, N2 = 8; };
-template <> struct Split<128, 1> { static constexpr int N1 = 8, N2 = 16; };
-template <> struct Split<64, 0> { static constexpr int N1 = 8, N2 = 8; };
-template <> struct Split<64, 1> { static constexpr int N1 = 8, N2 = 8; };
-
-// ---------------------------------------------------------------------------
-// column sweeps: tile of T consecutive kx, one column c, all N elements
-// ---------------------------------------------------------------------------
-template <int N, int T, int S = 0> struct Col2Cfg {
-  static constexpr int N1 = Split<N, S>::N1, N2 = Split<N, S>::N2;
-  static constexpr int NJ = N1 > N2 ? N1 : N2;
-  static constexpr int NT = T * NJ;
-  static constexpr int SR = N2 * T + 8;  // exchange row stride (+8: half-bank shift between rows)
-  static constexpr size_t SMEM = size_t(N1) * SR * sizeof(float2);
-  // at 810 the tile of 8 columns keeps 80 registers and three CTAs per SM
-  static constexpr int MINB = N == 810 ? (T == 4 ? 6 : (T == 8 ? 3 : 1)) : 1;
-};
-
-// DRV: the launch carries derivative outputs (ColArgs::ndrv > 0).  Without it
-// the wavenumber scaling is compiled out; otherwise the compiler hoists the
-// int -> double -> float conversions of every element out of the `drv` branch
-// and pays for them on the XU pipe even for plain components.
-// FULL: the transform axis has the 2/3-rule compact layout of the solver
-// (kpos = N/3 + 1, kneg = N/3), so which of each thread's N1 gathers (inverse)
-// or N2 stores (forward) touch a retained mode is known at compile time except
-// in the one block that straddles a boundary; the unused forward outputs are
-// then never formed.
-template <int N, int T, bool INV, bool DRV, bool FULL, int S = 0>
-__global__ void __launch_bounds__(Col2Cfg<N, T, S>::NT, Col2Cfg<N, T, S>::MINB)
-k_col2(const ColArgs a, const float2* __restrict__ tw) {
-  using C = float2;
-  using Cfg = Col2Cfg<N, T, S>;
-  constexpr int N1 = Cfg::N1, N2 = Cfg::N2, SR = Cfg::SR;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* ys = reinterpret_cast<C*>(smem_raw);
-  const int t = threadIdx.x % T, j = threadIdx.x / T;
-  const int kx = blockIdx.x * T + t;
-  const int c = blockIdx.y;
-  const int q = blockIdx.z;
-  const bool drv = DRV && q >= a.ncomp;
-  const C* __restrict__ in = static_cast<const C*>(a.in[drv ? a.drv_src[q - a.ncomp] : q]);
-  C* __restrict__ out = static_cast<C*>(a.out[q]);
-  const bool live = kx < a.K1;
-  constexpr int KP = N / 3 + 1, KN = N / 3;
-  const int kpos = FULL ? KP : a.kpos, kneg = FULL ? KN : a.kneg;
-  const int Kc = kpos + kneg;
-  // element offsets fit in 32 bits for every sweep (at most ~3.5e8 elements
-  // per component), so the per-element address arithmetic stays 32-bit
-  const int ies = int(a.in_es), oes = int(a.out_es);
-  if (j < N2) {
-    C v[N1];
-    const C* base = in + kx + (long long)c * a.in_cs;
-    if (INV) {
-#pragma unroll
-      for (int n1 = 0; n1 < N1; ++n1) {
-        const int e = N2 * n1 + j;
-        v[n1] = mk<C>(0.f, 0.f);
-        const int rg = FULL ? crange(N2 * n1, N2, N, KP, KN) : 3;
-        if (rg == 2) continue;
-        const int p = rg == 0 ? e : (rg == 1 ? e - N + Kc : cpos(e, N, kpos, kneg));
-        if (live && p >= 0 && !(a.zero_origin && kx == 0 && c == 0 && p == 0)) {
-          v[n1] = __ldg(base + p * ies);
-          if (drv) {
-            const float kk = float(a.kfac * double(p < kpos ? p : p - Kc));
-            v[n1] = mk<C>(-kk * v[n1].y, kk * v[n1].x);
-          }
-        }
-      }
-    } else {
-      const C* bj = base + j * ies;
-      const int st = N2 * ies;
-#pragma unroll
-      for (int n1 = 0; n1 < N1; ++n1) v[n1] = live ? __ldg(bj + n1 * st) : mk<C>(0.f, 0.f);
-    }
-    DFT<N1, INV, C>::run(v);
-#pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1) {
-      C w = __ldg(&tw[j * k1]);
-      if (INV) w.y = -w.y;
-      v[k1] = cmul(v[k1], w);
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) ys[k1 * SR + j * T + t] = v[k1];
-  }
-  __syncthreads();
-  if (j < N1 && live) {
-    C w[N2];
-#pragma unroll
-    for (int n2 = 0; n2 < N2; ++n2) w[n2] = ys[j * SR + n2 * T + t];
-    DFT<N2, INV, C>::run(w);
-    C* obase = out + kx + (long long)c * a.out_cs;
-    if (INV) {
-      C* oj = obase + j * oes;
-      const int st = N1 * oes;
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) oj[k2 * st] = w[k2];
-    } else {
-      // retained e = j + N1 k2: e < kpos keeps its index, e >= N - kneg moves down by N - Kc
-      const int shift = N - Kc;
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) {
-        const int e = j + N1 * k2;
-        const int rg = FULL ? crange(N1 * k2, N1, N, KP, KN) : 3;
-        if (rg == 0) obase[e * oes] = w[k2];
-        else if (rg == 1) obase[(e - shift) * oes] = w[k2];
-        else if (rg == 3) {
-          if (e < kpos) obase[e * oes] = w[k2];
-          else if (e >= N - kneg) obase[(e - shift) * oes] = w[k2];
-        }
-      }
-    }
-  }
-}
+// the two-level split of the CTA-wide x sweeps
+template <int N> struct Split;
+template <> struct Split<128> { static constexpr int N1 = 16, N2 = 8; };
+template <> struct Split<64> { static constexpr int N1 = 8, N2 = 8; };
 
 // ---------------------------------------------------------------------------
 // asynchronous global -> shared copies
@@ -814,8 +686,7 @@ template <typename F> static void set_smem2(F* f, size_t bytes) {
 }
 
 // Column-sweep variants the autotuner chooses from, per N: (tile width T,
-// split S).  Variant 0 is the default; launches with derivative outputs always
-// use variant 0.
+// split S).  Variant 0 is the default.
 template <int N> struct ColVariants;
 template <> struct ColVariants<810> {
   static constexpr int count = 4;
@@ -836,11 +707,11 @@ template <> struct ColVariants<64> {
 };
 
 template <int N, int T, int S> static void init_col2_variant() {
-  using Cfg = Col2Cfg<N, T, S>;
-  set_smem2(k_col2<N, T, true, false, false, S>, Cfg::SMEM);
-  set_smem2(k_col2<N, T, true, false, true, S>, Cfg::SMEM);
-  set_smem2(k_col2<N, T, false, false, false, S>, Cfg::SMEM);
-  set_smem2(k_col2<N, T, false, false, true, S>, Cfg::SMEM);
+  using Cfg = Col2Cfg<float, N, T, S>;
+  set_smem2(k_col2<float, N, T, true, false, S>, Cfg::SMEM);
+  set_smem2(k_col2<float, N, T, true, true, S>, Cfg::SMEM);
+  set_smem2(k_col2<float, N, T, false, false, S>, Cfg::SMEM);
+  set_smem2(k_col2<float, N, T, false, true, S>, Cfg::SMEM);
 }
 
 template <int N, int V = 0> static void init_col2_variants() {
@@ -851,9 +722,6 @@ template <int N, int V = 0> static void init_col2_variants() {
 }
 
 template <int N> static void init_fast_n() {
-  constexpr int T = ColVariants<N>::T[0];
-  set_smem2(k_col2<N, T, true, true, false>, Col2Cfg<N, T>::SMEM);
-  set_smem2(k_col2<N, T, true, true, true>, Col2Cfg<N, T>::SMEM);
   init_col2_variants<N>();
   if constexpr (N == 64 || N == 128) {
     set_smem2(k_xsweep3<N>, X3Cfg<N>::SMEM);
@@ -881,11 +749,11 @@ bool init_fast(int N) {
 // buffered tiles) in both directions (810^3 inverse y sweep, 81 planes:
 // 0.166 ms against 0.283 ms for a persistent three-level kernel).
 template <int N, int T, int S, bool INV> static void col2_launch(const ColArgs& a, const float2* t2, cudaStream_t st) {
-  using Cfg = Col2Cfg<N, T, S>;
+  using Cfg = Col2Cfg<float, N, T, S>;
   dim3 grid((a.K1 + T - 1) / T, a.ncols, a.ncomp);
   const bool full = a.kpos == N / 3 + 1 && a.kneg == N / 3;
-  if (full) k_col2<N, T, INV, false, true, S><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
-  else k_col2<N, T, INV, false, false, S><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
+  if (full) k_col2<float, N, T, INV, true, S><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
+  else k_col2<float, N, T, INV, false, S><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
 }
 
 template <int N, bool INV, int V = 0> static void col2_variant(int v, const ColArgs& a, const float2* t2,
@@ -898,17 +766,6 @@ template <int N, bool INV, int V = 0> static void col2_variant(int v, const ColA
 
 template <int N, bool INV> static void col2_n(const ColArgs& a, const void* tw, cudaStream_t st) {
   const float2* t2 = static_cast<const float2*>(tw);
-  if constexpr (INV) {
-    if (a.ndrv > 0) {
-      constexpr int T = ColVariants<N>::T[0];
-      using Cfg = Col2Cfg<N, T>;
-      dim3 grid((a.K1 + T - 1) / T, a.ncols, a.ncomp + a.ndrv);
-      const bool full = a.kpos == N / 3 + 1 && a.kneg == N / 3;
-      if (full) k_col2<N, T, true, true, true><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
-      else k_col2<N, T, true, true, false><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
-      return;
-    }
-  }
   if (N == 810 && a.variant >= kColTmaVariant && a.variant < kColTmaVariant + kColTmaConfigs &&
       launch_colt(N, INV, a, tw, a.variant - kColTmaVariant, st))
     return;

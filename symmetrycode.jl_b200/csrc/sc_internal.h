@@ -23,12 +23,6 @@ struct ColArgs {
   long long in_cs, in_es, out_cs, out_es;
   int kpos, kneg;     // compact mapping of the transform axis
   int zero_origin;    // inverse only: treat (kx, c, e) = (0, 0, 0) as zero (k = 0 mode)
-  // optional derivative outputs (inverse only): out[ncomp + j] = transform of
-  // (i * kfac * k_e) * in[deriv_src[j]] where k_e is the signed wavenumber of
-  // compact position e; ndrv = 0 disables
-  int ndrv;
-  int drv_src[kMaxComp];
-  double kfac;
   int variant;  // FP32 fast sizes: kernel variant chosen by the autotuner (0 = default)
   // bounded device waits of the TMA-fed sweeps: polls before a wait gives up
   // and the plan's device error word it then sets (nullptr: no TMA sweep)

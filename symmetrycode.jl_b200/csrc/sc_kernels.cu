@@ -15,6 +15,7 @@
 // zero modes `twothirds!` (src/solver.jl:371-389) would mask are never read.
 #include "sc_fft.cuh"
 #include "sc_internal.h"
+#include "sc_col.h"
 #include "sc_xrow.h"
 
 #include <cstdlib>
@@ -68,11 +69,8 @@ k_col_inv(const ColArgs a, const typename V2<R>::T* __restrict__ tw) {
   const int kx0 = blockIdx.x * T;
   const int c = blockIdx.y;
   const int q = blockIdx.z;
-  const bool drv = q >= a.ncomp;
-  const int src = drv ? a.drv_src[q - a.ncomp] : q;
-  const C* __restrict__ in = static_cast<const C*>(a.in[src]);
+  const C* __restrict__ in = static_cast<const C*>(a.in[q]);
   C* __restrict__ out = static_cast<C*>(a.out[q]);
-  const int Kc = a.kpos + a.kneg;
   // all loads of the tile are issued before the first shared-memory store so
   // that each thread keeps LPT requests in flight
   constexpr int LPT = (T * N + NT - 1) / NT;
@@ -90,16 +88,7 @@ k_col_inv(const ColArgs a, const typename V2<R>::T* __restrict__ tw) {
 #pragma unroll
   for (int i = 0; i < LPT; ++i) {
     const int idx = threadIdx.x + i * NT;
-    if (T * N % NT == 0 || idx < T * N) {
-      const int t = idx % T, e = idx / T;
-      C w = v[i];
-      if (drv) {  // multiply by i k_e
-        const int p = compact_pos(e, N, a.kpos, a.kneg);
-        const R kk = R(a.kfac * double(p < a.kpos ? p : p - Kc));
-        w = mk<C>(-kk * w.y, kk * w.x);
-      }
-      s[e * T + t] = w;
-    }
+    if (T * N % NT == 0 || idx < T * N) s[(idx / T) * T + idx % T] = v[i];
   }
   __syncthreads();
   tile_fft<C, N, T, NT, true, true>(s, tw);
@@ -751,7 +740,7 @@ __global__ void k_spectrum(const PackArgs a, int nshell, double* s) {
   X(90) X(96) X(120) X(128) X(160) X(180) X(192) X(240) X(256) X(270) X(320) X(360) X(384) X(512) X(540) \
   X(640) X(720) X(768) X(810) X(1024)
 
-// sizes whose x transforms run on the shared-memory engine; the others are those
+// sizes whose transforms run on the shared-memory engine; the others are those
 // of sc_sweep_sizes.h
 #define SC_SIZES_SMALL(X) X(4) X(6) X(8) X(10) X(12) X(16) X(18) X(20) X(24) X(30)
 
@@ -768,7 +757,7 @@ template <typename R, int N>
 static bool col_inv_n(const ColArgs& a, const void* tw, cudaStream_t st) {
   using C = typename V2<R>::T;
   using Cfg = ColCfg<R, N>;
-  dim3 grid((a.K1 + Cfg::T - 1) / Cfg::T, a.ncols, a.ncomp + a.ndrv);
+  dim3 grid((a.K1 + Cfg::T - 1) / Cfg::T, a.ncols, a.ncomp);
   k_col_inv<R, N><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, static_cast<const C*>(tw));
   return true;
 }
@@ -809,9 +798,9 @@ static bool xr2c_n(const XPlainArgs& a, const void* tw, cudaStream_t st) {
 }
 
 template <typename R, int N> static bool init_n() {
-  set_smem(k_col_inv<R, N>, ColCfg<R, N>::SMEM);
-  set_smem(k_col_fwd<R, N>, ColCfg<R, N>::SMEM);
   if constexpr (N < 32) {
+    set_smem(k_col_inv<R, N>, ColCfg<R, N>::SMEM);
+    set_smem(k_col_fwd<R, N>, ColCfg<R, N>::SMEM);
     set_smem(k_xsweep_ns<R, N, 2>, XCfg<R, N>::SMEM);
     set_smem(k_xsweep_ns<R, N, 3>, XCfg<R, N>::SMEM);
     set_smem(k_x_c2r<R, N>, XPCfg<R, N>::SMEM);
@@ -824,7 +813,7 @@ template <typename R, int N> static bool init_n() {
 // process and device, before any launch or stream capture).
 template <typename R> bool init_kernels(int N) {
   if (sizeof(R) == 4 && fast_supported(N) && !init_fast(N)) return false;
-  if (!xrow_init<R>(N)) return false;
+  if (!xrow_init<R>(N) || !col_init<R>(N)) return false;
   switch (N) {
 #define SC_CASE(NN) case NN: return init_n<R, NN>();
     SC_SIZES(SC_CASE)
@@ -839,18 +828,20 @@ template <typename R> static bool use_fast(int N) {
 
 template <typename R> bool launch_col_inv(int N, const ColArgs& a, const void* tw, cudaStream_t st) {
   if (use_fast<R>(N)) return launch_col2(N, true, a, tw, st);
+  if (col_sweep<R>(N, true, a, tw, st)) return true;
   switch (N) {
 #define SC_CASE(NN) case NN: return col_inv_n<R, NN>(a, tw, st);
-    SC_SIZES(SC_CASE)
+    SC_SIZES_SMALL(SC_CASE)
 #undef SC_CASE
     default: return false;
   }
 }
 template <typename R> bool launch_col_fwd(int N, const ColArgs& a, const void* tw, cudaStream_t st) {
   if (use_fast<R>(N)) return launch_col2(N, false, a, tw, st);
+  if (col_sweep<R>(N, false, a, tw, st)) return true;
   switch (N) {
 #define SC_CASE(NN) case NN: return col_fwd_n<R, NN>(a, tw, st);
-    SC_SIZES(SC_CASE)
+    SC_SIZES_SMALL(SC_CASE)
 #undef SC_CASE
     default: return false;
   }
