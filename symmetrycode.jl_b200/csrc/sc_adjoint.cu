@@ -20,11 +20,12 @@ struct Mode {
   int ix, iy, iz;
   bool origin;
 };
-__device__ __forceinline__ Mode dmode(long long i, int kc, int D) {
+__device__ __forceinline__ Mode dmode(long long i64, int kc, int D) {
+  const unsigned i = unsigned(i64);  // fewer than 2^31 modes at every size: 32-bit divisions
   const int K1 = kc + 1, K2 = 2 * kc + 1;
   Mode m;
-  m.ix = int(i % K1);
-  const long long r = i / K1;
+  const unsigned r = i / K1;
+  m.ix = int(i - r * K1);
   const int py = int(r % K2), pz = D == 3 ? int(r / K2) : 0;
   m.iy = py <= kc ? py : py - K2;
   m.iz = pz <= kc ? pz : pz - K2;
@@ -163,7 +164,7 @@ __global__ void k_mse(CPtr3 u, CPtr3 t, Ptr3 g, double coef, int D, int kc, doub
   const long long nm = (long long)K1 * K2 * (D == 3 ? K2 : 1);
   double acc = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nm; i += (long long)gridDim.x * blockDim.x) {
-    const double w = (i % K1) == 0 ? 1.0 : 2.0;
+    const double w = unsigned(i) % unsigned(K1) == 0 ? 1.0 : 2.0;
     for (int c = 0; c < D; ++c) {
       const C a = static_cast<const C*>(u.p[c])[i], b = static_cast<const C*>(t.p[c])[i];
       const double dx = double(a.x) - double(b.x), dy = double(a.y) - double(b.y);

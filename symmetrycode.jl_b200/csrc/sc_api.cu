@@ -71,6 +71,7 @@ struct sc_plan {
   void* cc[3] = {};
   void* dd[6] = {};
   double* dscal = nullptr;  // [0] forcing A, [1] reduction accumulator
+  double* shells = nullptr;  // kc + 3 shell sums of the spectrum and the diagnostics
   int* err = nullptr;       // device word set when a bounded wait of a TMA-fed sweep ran out
   void* fa = nullptr, *fb = nullptr;  // full-spectrum scratch (lazy)
   std::vector<void*> allocs;
@@ -1103,6 +1104,7 @@ int sc_plan_create(sc_plan** out, int D, int n, double l, int dtype, size_t* wor
   for (int c = 0; c < D; ++c)
     if ((rc = plan_alloc(p, &p->cc[c], plane * p->esz))) goto bad;
   if ((rc = plan_alloc(p, (void**)&p->dscal, 16 * sizeof(double)))) goto bad;
+  if ((rc = plan_alloc(p, (void**)&p->shells, (p->kc + 3) * sizeof(double)))) goto bad;
   if ((rc = plan_alloc(p, (void**)&p->err, sizeof(int)))) goto bad;
   if (cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking) != cudaSuccess) {
     rc = fail(SC_ERR_CUDA, "stream creation failed");
@@ -2000,20 +2002,22 @@ int clamp_impl(sc_plan* p, void* const* uc, double* eref_host, int mode, cudaStr
   return SC_OK;
 }
 
+// u: the compact state, or the full layout when `full`.  The shell sums live in
+// the plan: a stream-ordered buffer per call cost more than the sums (the pool
+// gives its memory back at every synchronisation).
 template <typename R>
-int spectrum_impl(sc_plan* p, void* const* uc, int nshell, double* out, cudaStream_t st) {
-  double* d = nullptr;
-  SC_CU(cudaMallocAsync((void**)&d, nshell * sizeof(double), st));
-  cudaMemsetAsync(d, 0, nshell * sizeof(double), st);
+int spectrum_impl(sc_plan* p, const void* const* u, int nshell, double* out, cudaStream_t st, bool full) {
+  double* d = p->shells;
+  SC_CU(cudaMemsetAsync(d, 0, nshell * sizeof(double), st));
   sc::PackArgs a{};
-  for (int c = 0; c < p->D; ++c) a.src[c] = uc[c];
+  for (int c = 0; c < p->D; ++c) a.src[c] = u[c];
   a.ncomp = p->D; a.D = p->D; a.n = p->n; a.kc = p->kc;
-  sc::launch_spectrum<R>(a, nshell, d, st);
+  sc::launch_spectrum<R>(a, nshell, d, st, full);
   int rc = check_launch("spectrum");
-  cudaMemcpyAsync(out, d, nshell * sizeof(double), cudaMemcpyDeviceToHost, st);
-  cudaFreeAsync(d, st);
+  if (rc) return rc;
+  SC_CU(cudaMemcpyAsync(out, d, nshell * sizeof(double), cudaMemcpyDeviceToHost, st));
   SC_CU(cudaStreamSynchronize(st));
-  return rc;
+  return SC_OK;
 }
 }  // namespace
 
@@ -2077,9 +2081,7 @@ int sc_spectrum(sc_plan* p, const void* const* u, int nshell, double* s, void* s
   if (!rc) rc = ensure_device(p);
   if (rc) return rc;
   cudaStream_t st = as_stream(stream);
-  rc = SC_DTYPE_DISPATCH(p, pack_state, p, u, p->S, st);
-  if (rc) return rc;
-  return SC_DTYPE_DISPATCH(p, spectrum_impl, p, p->S, nshell, s, st);
+  return SC_DTYPE_DISPATCH(p, spectrum_impl, p, u, nshell, s, st, true);
 }
 
 int sc_les_diagnostics(sc_plan* p, sc_closure* cl, const void* const* u, const void* const* uref, double visc,
@@ -2101,12 +2103,10 @@ int sc_les_diagnostics(sc_plan* p, sc_closure* cl, const void* const* u, const v
     out[1] = 0.5 * s;
     if ((r = energy_impl<R>(p, u, 0, 1, &s, st))) return r;
     out[2] = visc * s;
-    if ((r = pack_state<R>(p, u, p->S, st))) return r;
-    if ((r = spectrum_impl<R>(p, p->S, nshell, spec, st))) return r;
-    // e_post and the closure terms accumulate into dscal[1..2] and a shell buffer
-    double* d = nullptr;
-    SC_CU(cudaMallocAsync((void**)&d, (3 + nshell) * sizeof(double), st));
-    cudaMemsetAsync(d, 0, (3 + nshell) * sizeof(double), st);
+    if ((r = spectrum_impl<R>(p, u, nshell, spec, st, true))) return r;
+    // e_post and the closure terms accumulate into the plan's shell buffer
+    double* d = p->shells;
+    SC_CU(cudaMemsetAsync(d, 0, (3 + nshell) * sizeof(double), st));
     sc::DiagArgs a{};
     a.D = p->D; a.n = p->n; a.kc = p->kc; a.kfac = 2.0 * M_PI / p->l;
     for (int c = 0; c < p->D; ++c) a.u[c] = u[c];
@@ -2115,8 +2115,9 @@ int sc_les_diagnostics(sc_plan* p, sc_closure* cl, const void* const* u, const v
       sc::launch_epost<R>(a, d, st);
     }
     if (cl) {
-      if ((r = products<R>(p, p->S, st))) { cudaFreeAsync(d, st); return r; }
-      if ((r = closure_tauhat<R>(cl, p->S, st))) { cudaFreeAsync(d, st); return r; }
+      if ((r = pack_state<R>(p, u, p->S, st))) return r;
+      if ((r = products<R>(p, p->S, st))) return r;
+      if ((r = closure_tauhat<R>(cl, p->S, st))) return r;
       sc::DiagArgs b = a;
       for (int c = 0; c < p->D; ++c) b.u[c] = p->S[c];
       for (int c = 0; c < (p->D == 3 ? 6 : 3); ++c) b.th[c] = cl->th[c];
@@ -2124,8 +2125,7 @@ int sc_les_diagnostics(sc_plan* p, sc_closure* cl, const void* const* u, const v
     }
     r = check_launch("les diagnostics");
     std::vector<double> h(3 + nshell);
-    cudaMemcpyAsync(h.data(), d, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(d, st);
+    SC_CU(cudaMemcpyAsync(h.data(), d, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     SC_CU(cudaStreamSynchronize(st));
     if (r) return r;
     out[0] = uref ? std::sqrt(h[0]) / std::sqrt(h[1]) : 0.0;

@@ -39,6 +39,26 @@ constexpr int crange(int e0, int B, int N, int kpos, int kneg) {
 }
 
 // ---------------------------------------------------------------------------
+// division of indexes below 2^31 by a run-time extent: multiply-high and shift
+// (round-up method of Granlund and Montgomery, "Division by invariant integers
+// using multiplication", 1994) instead of the 64-bit division subroutine
+// ---------------------------------------------------------------------------
+struct FastDiv {
+  unsigned d = 1, m = 0, s = 0;
+  FastDiv() = default;
+  explicit FastDiv(int div) : d(unsigned(div)) {
+    while ((1ull << s) < d) ++s;
+    m = unsigned(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+  }
+  __device__ __forceinline__ unsigned div(unsigned x) const { return (__umulhi(m, x) + x) >> s; }
+  __device__ __forceinline__ unsigned divmod(unsigned x, unsigned& r) const {
+    const unsigned q = div(x);
+    r = x - q * d;
+    return q;
+  }
+};
+
+// ---------------------------------------------------------------------------
 // complex helpers
 // ---------------------------------------------------------------------------
 template <typename R> struct V2;

@@ -114,7 +114,9 @@ template <typename R> bool launch_x_vmax(int N, const XPlainArgs& a, const void*
                                          cudaStream_t st);
 // shells 1..2 on the compact state held in a.dst: mode 0 measures into eref[0..1], mode 1 rescales
 template <typename R> void launch_shell_clamp(const PackArgs& a, double* eref, int mode, cudaStream_t st);
-template <typename R> void launch_spectrum(const PackArgs& a, int nshell, double* s, cudaStream_t st);
+// a.src: the compact cube, or the full RFFT layout when `full`; adds into s
+template <typename R>
+void launch_spectrum(const PackArgs& a, int nshell, double* s, cudaStream_t st, bool full = false);
 template <typename R> void launch_pack(const PackArgs& a, cudaStream_t st);
 template <typename R> void launch_unpack(const PackArgs& a, cudaStream_t st);
 // forcing coefficient A = eps / (2 E_band) of the compact state u into *A

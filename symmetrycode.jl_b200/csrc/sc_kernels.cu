@@ -341,15 +341,15 @@ k_x_r2c(const XPlainArgs a, const typename V2<R>::T* __restrict__ tw) {
 // out_a    = base_a + ca k   (projected when proj_a: wray3!, :992-1001)
 // out_b    = base_b + cb k
 template <typename R, int D>
-__global__ void __launch_bounds__(256) k_epilogue(const EpiArgs a) {
+__global__ void __launch_bounds__(256) k_epilogue(const EpiArgs a, const FastDiv dx, const FastDiv dy) {
   using C = typename V2<R>::T;
-  const long long nm = (long long)a.K1 * a.K2 * (D == 3 ? a.K2 : 1);
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  // fewer than 2^31 modes at every size: 32-bit index arithmetic
+  const unsigned nm = unsigned(a.K1) * a.K2 * (D == 3 ? a.K2 : 1);
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nm) return;
-  const int ix = int(i % a.K1);
-  const long long r = i / a.K1;
-  const int py = int(r % a.K2);
-  const int pz = D == 3 ? int(r / a.K2) : 0;
+  unsigned ux, uy;
+  const unsigned uz = dy.divmod(dx.divmod(i, ux), uy);
+  const int ix = int(ux), py = int(uy), pz = D == 3 ? int(uz) : 0;
   const int iky = py <= a.kc ? py : py - a.K2;
   const int ikz = pz <= a.kc ? pz : pz - a.K2;
   const R kf = R(a.kfac);
@@ -443,11 +443,11 @@ template <typename R, int D>
 __global__ void k_filter(const FilterArgs a) {
   using C = typename V2<R>::T;
   const int K1 = a.kcl + 1, K2 = 2 * a.kcl + 1;
-  const long long nm = (long long)K1 * K2 * (D == 3 ? K2 : 1);
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned nm = unsigned(K1) * K2 * (D == 3 ? K2 : 1);
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nm) return;
-  const int ix = int(i % K1);
-  const long long r = i / K1;
+  const unsigned r = i / K1;
+  const int ix = int(i - r * K1);
   const int py = int(r % K2);
   const int pz = D == 3 ? int(r / K2) : 0;
   const int iy = py <= a.kcl ? py : py - K2;
@@ -489,43 +489,58 @@ __global__ void k_filter(const FilterArgs a) {
 // ---------------------------------------------------------------------------
 // pack / unpack between the full RFFT layout and the compact 2/3 cube
 // ---------------------------------------------------------------------------
+// Both are bound by memory; a block takes kPackSpan consecutive elements of one
+// z plane, so an index costs one multiply-high (64-bit divisions and one element
+// a thread: unpack 3.87 ms at 810^3 FP32, three components).
+constexpr int kPackThreads = 256, kPackPer = 4, kPackSpan = kPackThreads * kPackPer;
+
 template <typename R>
-__global__ void k_pack(const PackArgs a) {
+__global__ void __launch_bounds__(kPackThreads) k_pack(const PackArgs a, const FastDiv dx) {
   using C = typename V2<R>::T;
   const int K1 = a.kc + 1, K2 = 2 * a.kc + 1, Kf = a.n / 2 + 1;
-  const long long nm = (long long)K1 * K2 * (a.D == 3 ? K2 : 1);
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nm) return;
-  const int ix = int(i % K1);
-  const long long r = i / K1;
-  const int py = int(r % K2);
-  const int pz = a.D == 3 ? int(r / K2) : 0;
-  const int fy = py <= a.kc ? py : py + a.n - K2;
+  const unsigned nm = unsigned(K1) * K2;
+  const int pz = blockIdx.y;
   const int fz = pz <= a.kc ? pz : pz + a.n - K2;
-  const long long j = ix + (long long)Kf * (fy + (long long)a.n * fz);
-  const C* src = static_cast<const C*>(a.src[blockIdx.y]);
-  static_cast<C*>(a.dst[blockIdx.y])[i] = src[j];
+  const C* src = static_cast<const C*>(a.src[blockIdx.z]) + (long long)fz * a.n * Kf;
+  C* dst = static_cast<C*>(a.dst[blockIdx.z]) + (long long)pz * nm;
+  const unsigned i0 = blockIdx.x * kPackSpan + threadIdx.x;
+  C v[kPackPer];
+#pragma unroll
+  for (int u = 0; u < kPackPer; ++u) {
+    const unsigned i = i0 + u * kPackThreads;
+    unsigned ix;
+    const int py = int(dx.divmod(i, ix));
+    const int fy = py <= a.kc ? py : py + a.n - K2;
+    if (i < nm) v[u] = __ldg(src + fy * Kf + ix);
+  }
+#pragma unroll
+  for (int u = 0; u < kPackPer; ++u)
+    if (i0 + u * kPackThreads < nm) dst[i0 + u * kPackThreads] = v[u];
 }
 
 template <typename R>
-__global__ void k_unpack(const PackArgs a) {
+__global__ void __launch_bounds__(kPackThreads) k_unpack(const PackArgs a, const FastDiv dx) {
   using C = typename V2<R>::T;
   const int K1 = a.kc + 1, K2 = 2 * a.kc + 1, Kf = a.n / 2 + 1;
-  const long long nm = (long long)Kf * a.n * (a.D == 3 ? a.n : 1);
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nm) return;
-  const int ix = int(j % Kf);
-  const long long r = j / Kf;
-  const int fy = int(r % a.n);
-  const int fz = a.D == 3 ? int(r / a.n) : 0;
-  const int py = compact_pos(fy, a.n, a.kc + 1, a.kc);
-  const int pz = a.D == 3 ? compact_pos(fz, a.n, a.kc + 1, a.kc) : 0;
-  C v = mk<C>(R(0), R(0));
-  if (ix < K1 && py >= 0 && pz >= 0) {
-    const long long i = ix + (long long)K1 * (py + (long long)K2 * pz);
-    v = static_cast<const C*>(a.src[blockIdx.y])[i];
+  const unsigned nm = unsigned(Kf) * a.n;
+  const int fz = blockIdx.y;
+  const int pz = compact_pos(fz, a.n, a.kc + 1, a.kc);
+  const C* src = static_cast<const C*>(a.src[blockIdx.z]) + (long long)(a.D == 3 ? pz : 0) * K1 * K2;
+  C* dst = static_cast<C*>(a.dst[blockIdx.z]) + (long long)fz * nm;
+  const unsigned j0 = blockIdx.x * kPackSpan + threadIdx.x;
+  C v[kPackPer];
+#pragma unroll
+  for (int u = 0; u < kPackPer; ++u) {
+    const unsigned j = j0 + u * kPackThreads;
+    unsigned ux;
+    const int fy = int(dx.divmod(j, ux)), ix = int(ux);
+    const int py = compact_pos(fy, a.n, a.kc + 1, a.kc);
+    v[u] = mk<C>(R(0), R(0));
+    if (j < nm && ix < K1 && py >= 0 && pz >= 0) v[u] = __ldg(src + py * K1 + ix);
   }
-  static_cast<C*>(a.dst[blockIdx.y])[j] = v;
+#pragma unroll
+  for (int u = 0; u < kPackPer; ++u)
+    if (j0 + u * kPackThreads < nm) dst[j0 + u * kPackThreads] = v[u];
 }
 
 // ---------------------------------------------------------------------------
@@ -580,13 +595,14 @@ template <typename R>
 __global__ void k_spectral_energy(const PackArgs a, int K1, int K2, int compact, double kfac, int weight_k2,
                                   double* out, int mask23) {
   using C = typename V2<R>::T;
-  const long long nm = (long long)K1 * K2 * (a.D == 3 ? K2 : 1);
+  const unsigned nm = unsigned(K1) * K2 * (a.D == 3 ? K2 : 1);  // < 2^31 at every size
   double e = 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nm; i += (long long)gridDim.x * blockDim.x) {
-    const int ix = int(i % K1);
+#pragma unroll 4
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nm; i += gridDim.x * blockDim.x) {
+    const unsigned r = i / K1;
+    const int ix = int(i - r * K1);
     double w = (ix == 0 || (!compact && 2 * ix == a.n)) ? 1.0 : 2.0;
     if (weight_k2 || mask23) {
-      const long long r = i / K1;
       const int py = int(r % K2);
       const int pz = a.D == 3 ? int(r / K2) : 0;
       int iky, ikz;
@@ -707,29 +723,55 @@ __global__ void k_shell_clamp(const PackArgs a, double* eref, int mode) {
   }
 }
 
-// spectrum (src/solver.jl:693-699): s[i-1] += 1/2 sum over modes with i <= |k| < i+1 (RFFT double count)
-template <typename R>
-__global__ void k_spectrum(const PackArgs a, int nshell, double* s) {
+// spectrum (src/solver.jl:693-699): s[i-1] += 1/2 sum over modes with i <= |k| < i+1 (RFFT double count),
+// from the compact cube or straight from the full RFFT layout (FULL).  One warp
+// per (ky, kz) row: the shell grows along the row, so equal shells are runs of
+// neighbouring lanes; a segmented shuffle sums each run and its first lane adds
+// to the block's bins in shared memory.  (One global atomic per mode on nshell
+// addresses took 338 us at 256^3.)
+template <typename R, bool FULL>
+__global__ void __launch_bounds__(256) k_spectrum(const PackArgs a, int nshell, double* s) {
   using C = typename V2<R>::T;
-  const int K1 = a.kc + 1, K2 = 2 * a.kc + 1;
-  const long long nm = (long long)K1 * K2 * (a.D == 3 ? K2 : 1);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nm; i += (long long)gridDim.x * blockDim.x) {
-    const int ix = int(i % K1);
-    const long long r = i / K1;
-    const int py = int(r % K2), pz = a.D == 3 ? int(r / K2) : 0;
+  extern __shared__ double bins[];
+  for (int i = threadIdx.x; i < nshell; i += blockDim.x) bins[i] = 0.0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, K2 = 2 * a.kc + 1;
+  const int nrow = K2 * (a.D == 3 ? K2 : 1);
+  const int kmax = min(a.kc, nshell);  // |k| < nshell + 1 needs kx <= nshell
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrow; r += (gridDim.x * blockDim.x) >> 5) {
+    const int py = r % K2, pz = a.D == 3 ? r / K2 : 0;
     const int iy = py <= a.kc ? py : py - K2, iz = pz <= a.kc ? pz : pz - K2;
-    const long long k2 = (long long)ix * ix + (long long)iy * iy + (long long)iz * iz;
-    int sh = int(sqrt(double(k2)));
-    while ((long long)(sh + 1) * (sh + 1) <= k2) ++sh;
-    while ((long long)sh * sh > k2) --sh;
-    if (sh < 1 || sh > nshell) continue;
-    double e = 0;
-    for (int c = 0; c < a.D; ++c) {
-      const C v = static_cast<const C*>(a.src[c])[i];
-      e += double(v.x) * v.x + double(v.y) * v.y;
+    const int q2 = iy * iy + iz * iz;
+    if (q2 >= (nshell + 1) * (nshell + 1)) continue;  // whole warps
+    const long long base = FULL ? (long long)(a.n / 2 + 1) * ((iy < 0 ? iy + a.n : iy) + (long long)a.n * (iz < 0 ? iz + a.n : iz))
+                                : (long long)(a.kc + 1) * r;
+    for (int x0 = 0; x0 <= kmax; x0 += 32) {
+      const int ix = x0 + lane;
+      const int k2 = q2 + ix * ix;
+      int sh = int(sqrtf(float(k2)));
+      while ((sh + 1) * (sh + 1) <= k2) ++sh;
+      while (sh * sh > k2) --sh;
+      double e = 0;
+      if (ix <= kmax && sh >= 1 && sh <= nshell) {
+        for (int c = 0; c < a.D; ++c) {
+          const C v = static_cast<const C*>(a.src[c])[base + ix];
+          e += double(v.x) * v.x + double(v.y) * v.y;
+        }
+        e *= ix > 0 ? 1.0 : 0.5;
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double e2 = __shfl_down_sync(0xffffffffu, e, o);
+        const int s2 = __shfl_down_sync(0xffffffffu, sh, o);
+        if (lane + o < 32 && s2 == sh) e += e2;
+      }
+      const int before = __shfl_up_sync(0xffffffffu, sh, 1);
+      if ((lane == 0 || before != sh) && sh >= 1 && sh <= nshell && e != 0.0) atomicAdd(&bins[sh - 1], e);
     }
-    atomicAdd(&s[sh - 1], 0.5 * (ix > 0 ? 2.0 : 1.0) * e);
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nshell; i += blockDim.x)
+    if (bins[i] != 0.0) atomicAdd(&s[i], bins[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -909,30 +951,32 @@ template <typename R> void launch_shell_clamp(const PackArgs& a, double* eref, i
   k_shell_clamp<R><<<1, 96, 0, st>>>(a, eref, mode);
 }
 
-template <typename R> void launch_spectrum(const PackArgs& a, int nshell, double* s, cudaStream_t st) {
-  const long long nm = (long long)(a.kc + 1) * (2 * a.kc + 1) * (a.D == 3 ? (2 * a.kc + 1) : 1);
-  long long nb = (nm + 255) / 256;
-  if (nb > 148 * 8) nb = 148 * 8;
-  k_spectrum<R><<<unsigned(nb), 256, 0, st>>>(a, nshell, s);
+template <typename R> void launch_spectrum(const PackArgs& a, int nshell, double* s, cudaStream_t st, bool full) {
+  const int K2 = 2 * a.kc + 1, nrow = K2 * (a.D == 3 ? K2 : 1);
+  int nb = (nrow + 7) / 8;  // eight rows a block
+  if (nb > 148 * 4) nb = 148 * 4;
+  const size_t sm = nshell * sizeof(double);
+  if (full) k_spectrum<R, true><<<nb, 256, sm, st>>>(a, nshell, s);
+  else k_spectrum<R, false><<<nb, 256, sm, st>>>(a, nshell, s);
 }
 
 template <typename R> void launch_epilogue(const EpiArgs& a, cudaStream_t st) {
   const long long nm = (long long)a.K1 * a.K2 * (a.D == 3 ? a.K2 : 1);
   const unsigned nb = unsigned((nm + 255) / 256);
-  if (a.D == 3) k_epilogue<R, 3><<<nb, 256, 0, st>>>(a);
-  else k_epilogue<R, 2><<<nb, 256, 0, st>>>(a);
+  const FastDiv dx(a.K1), dy(a.K2);
+  if (a.D == 3) k_epilogue<R, 3><<<nb, 256, 0, st>>>(a, dx, dy);
+  else k_epilogue<R, 2><<<nb, 256, 0, st>>>(a, dx, dy);
 }
 
 template <typename R> void launch_pack(const PackArgs& a, cudaStream_t st) {
   const int K1 = a.kc + 1, K2 = 2 * a.kc + 1;
-  const long long nm = (long long)K1 * K2 * (a.D == 3 ? K2 : 1);
-  dim3 grid(unsigned((nm + 255) / 256), a.ncomp);
-  k_pack<R><<<grid, 256, 0, st>>>(a);
+  const dim3 grid(unsigned((K1 * K2 + kPackSpan - 1) / kPackSpan), a.D == 3 ? K2 : 1, a.ncomp);
+  k_pack<R><<<grid, kPackThreads, 0, st>>>(a, FastDiv(K1));
 }
 template <typename R> void launch_unpack(const PackArgs& a, cudaStream_t st) {
-  const long long nm = (long long)(a.n / 2 + 1) * a.n * (a.D == 3 ? a.n : 1);
-  dim3 grid(unsigned((nm + 255) / 256), a.ncomp);
-  k_unpack<R><<<grid, 256, 0, st>>>(a);
+  const int Kf = a.n / 2 + 1;
+  const dim3 grid(unsigned((Kf * a.n + kPackSpan - 1) / kPackSpan), a.D == 3 ? a.n : 1, a.ncomp);
+  k_unpack<R><<<grid, kPackThreads, 0, st>>>(a, FastDiv(Kf));
 }
 template <typename R> void launch_band_forcing(const void* const* u, int D, int K1, int K2, int kc,
                                                double eps, double* A, cudaStream_t st) {
@@ -971,11 +1015,11 @@ template <typename R>
 __global__ void k_twothirds_full(const PackArgs a) {
   using C = typename V2<R>::T;
   const int Kf = a.n / 2 + 1;
-  const long long nm = (long long)Kf * a.n * (a.D == 3 ? a.n : 1);
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned nm = unsigned(Kf) * a.n * (a.D == 3 ? a.n : 1);  // < 2^31 at every size
+  const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nm) return;
-  const int ix = int(j % Kf);
-  const long long r = j / Kf;
+  const unsigned r = j / Kf;
+  const int ix = int(j - r * Kf);
   const int fy = int(r % a.n);
   const int fz = a.D == 3 ? int(r / a.n) : 0;
   const int ky = fy < a.n / 2 ? fy : fy - a.n;
@@ -990,11 +1034,11 @@ template <typename R>
 __global__ void k_project_full(const PackArgs a, double kfac) {
   using C = typename V2<R>::T;
   const int Kf = a.n / 2 + 1;
-  const long long nm = (long long)Kf * a.n * (a.D == 3 ? a.n : 1);
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned nm = unsigned(Kf) * a.n * (a.D == 3 ? a.n : 1);  // < 2^31 at every size
+  const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nm) return;
-  const int ix = int(j % Kf);
-  const long long r = j / Kf;
+  const unsigned r = j / Kf;
+  const int ix = int(j - r * Kf);
   const int fy = int(r % a.n);
   const int fz = a.D == 3 ? int(r / a.n) : 0;
   const R k[3] = {R(kfac * ix), R(kfac * (fy < a.n / 2 ? fy : fy - a.n)),
@@ -1041,7 +1085,7 @@ template <typename R> void launch_project_full(const PackArgs& a, double kfac, c
   template void launch_filter<R>(const FilterArgs&, cudaStream_t);                                   \
   template bool launch_x_vmax<R>(int, const XPlainArgs&, const void*, unsigned long long*, cudaStream_t); \
   template void launch_shell_clamp<R>(const PackArgs&, double*, int, cudaStream_t);                   \
-  template void launch_spectrum<R>(const PackArgs&, int, double*, cudaStream_t);
+  template void launch_spectrum<R>(const PackArgs&, int, double*, cudaStream_t, bool);
 SC_INST(float)
 SC_INST(double)
 

@@ -17,11 +17,12 @@ struct Modes {
   bool origin;
 };
 
-__device__ __forceinline__ Modes decode(long long i, int kc, int D) {
+__device__ __forceinline__ Modes decode(long long i64, int kc, int D) {
+  const unsigned i = unsigned(i64);  // fewer than 2^31 modes at every size: 32-bit divisions
   const int K1 = kc + 1, K2 = 2 * kc + 1;
   Modes m;
-  m.ix = int(i % K1);
-  const long long r = i / K1;
+  const unsigned r = i / K1;
+  m.ix = int(i - r * K1);
   const int py = int(r % K2);
   const int pz = D == 3 ? int(r / K2) : 0;
   m.iy = py <= kc ? py : py - K2;
