@@ -34,92 +34,12 @@
 #include <stdint.h>
 
 #include "sc_cnn.h"
+#include "sc_tcgen05.cuh"
+#include "sc_wgrad.h"
 
 namespace sc {
 
 namespace {
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  // UMMA shared-memory descriptor, K-major, no swizzle (layout type 0), version 1
-  uint64_t d = 0;
-  d |= uint64_t((saddr >> 4) & 0x3FFF);
-  d |= uint64_t((lbo >> 4) & 0x3FFF) << 16;
-  d |= uint64_t((sbo >> 4) & 0x3FFF) << 32;
-  d |= uint64_t(1) << 46;
-  return d;
-}
-
-template <int NOUT, bool F16 = false>
-__host__ __device__ constexpr uint32_t make_idesc() {
-  // kind::f16: D f32 (bits 4-5 = 1); A and B of one type, both bf16 (bits 7-9
-  // and 10-12 = 1) or both f16 (0); both K-major, N >> 3 at bit 17, M >> 4 at
-  // bit 24 (M = 128)
-  constexpr uint32_t ab = F16 ? 0u : 1u;
-  return (1u << 4) | (ab << 7) | (ab << 10) | (uint32_t(NOUT >> 3) << 17) | (uint32_t(128 >> 4) << 24);
-}
-
-// D += A B (the accumulators are zeroed in tensor memory beforehand), no lanes masked
-__device__ __forceinline__ void mma_bf16_acc(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-      :
-      : "r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(1u));
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
-// Polls the mbarrier phase `parity` at most `limit` times (try_wait suspends
-// for a hardware-defined time per poll); false when the wait ran out.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit) {
-  const uint32_t a = smem_u32(bar);
-  for (long long it = 0; it < limit; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-
-template <int NCOL>
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, float* v);
-
-template <>
-__device__ __forceinline__ void tmem_ld<16>(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// zero 32 lanes x 16 columns of tensor memory (this warp's lane quadrant)
-__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
-  const uint32_t z = 0;
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
-      "r"(z)
-      : "memory");
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
 
 // GELU in the tanh form of NNlib's gelu (the activation of the reference's nets):
 // 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3))).  The hardware tanh.approx
@@ -660,123 +580,6 @@ __global__ void k_gin_planar(const float* __restrict__ gin, const GinPtrs o, lon
   o.p[0][i] = v.x; o.p[1][i] = v.y; o.p[2][i] = v.z; o.p[3][i] = v.w;
 }
 
-// Weight and bias gradients of one layer (CUDA cores, FP32 accumulation,
-// FP64 atomics into the flat parameter gradient):
-//   gw[co][ci][t] += sum_v g[v][co] a[v + off(t)][ci],  gb[co] += sum_v g[v][co]
-// for co < cout, ci < cin.  Block (tap t, chunk of voxels).  Only the first CI
-// (4 | 32) input and CO (8 | 32) output channels are formed, the layer's own
-// channels rounded up to the tile, not the padded CP, COP of the activations.
-// A group of (CO/8)(CI/4) threads holds 8 x 4 (co, ci) register tiles, so a
-// voxel costs three 16-byte shared loads per 32 FMAs; the groups split each
-// staged block of VS voxels.  The bias sums run only in the centre-tap blocks.
-// The groups' tiles are summed in shared memory by all threads, then one FP64
-// atomic per gradient entry and block.
-// SPLIT: g = g + glo (BF16 high and low parts) and a = FP16 high + low parts
-// (a and alo of type __half); otherwise a is BF16 and glo, alo are unused.
-template <int KN, int CP, int COP, int CI, int CO, bool SPLIT>
-__global__ void __launch_bounds__(256)
-k_conv_wgrad(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ glo, const void* __restrict__ a,
-             const void* __restrict__ alo, int cin, int cout, int vchunk, double* __restrict__ gw,
-             double* __restrict__ gb) {
-  static_assert(CI % 4 == 0 && CI <= CP && CO % 8 == 0 && CO <= COP, "tile shape");
-  constexpr int TCO = 8, TCI = 4, NE = TCO * TCI;
-  constexpr int TG = (CO / TCO) * (CI / TCI);  // threads per group
-  constexpr int NG = 256 / TG;                  // groups
-  constexpr int VS = 128;                       // voxels per stage
-  constexpr int LG = CO + 4, LA = CI + 4;       // padded shared rows (16-byte multiples)
-  constexpr int STAGE = VS * (LG + LA);         // floats of one staged block
-  constexpr int RED = 256 * NE;                 // floats of the groups' tiles
-  constexpr long long NPTS = (long long)KN * KN * KN;
-  __shared__ __align__(16) float sbuf[STAGE > RED ? STAGE : RED];
-  float* sg = sbuf;            // [VS][LG]
-  float* sa = sbuf + VS * LG;  // [VS][LA]
-  const int t = blockIdx.x;    // tap
-  const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-  const bool centre = t == 13;
-  const int tid = threadIdx.x, grp = tid / TG, lt = tid % TG;
-  const int co0 = TCO * (lt / (CI / TCI)), ci0 = TCI * (lt % (CI / TCI));
-  float acc[TCO][TCI] = {};
-  float accb[TCO] = {};
-  const long long v0 = (long long)blockIdx.y * vchunk;
-  const long long v1 = min(v0 + vchunk, NPTS);
-  for (long long vb = v0; vb < v1; vb += VS) {
-    // stage the g rows and the shifted a rows (16-bit pairs -> FP32)
-    for (int i = tid; i < VS * CO / 2; i += 256) {
-      const int vv = i / (CO / 2), c = 2 * (i % (CO / 2));
-      const long long v = vb + vv;
-      float2 f = make_float2(0.f, 0.f);
-      if (v < v1) {
-        f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(g + v * COP + c));
-        if (SPLIT) {
-          const float2 l = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(glo + v * COP + c));
-          f.x += l.x; f.y += l.y;
-        }
-      }
-      *reinterpret_cast<float2*>(sg + vv * LG + c) = f;
-    }
-    for (int i = tid; i < VS * CI / 2; i += 256) {
-      const int vv = i / (CI / 2), c = 2 * (i % (CI / 2));
-      const long long v = vb + vv;
-      float2 f = make_float2(0.f, 0.f);
-      if (v < v1) {
-        const int x = int(v % KN), y = int((v / KN) % KN), z = int(v / ((long long)KN * KN));
-        const long long q = ((long long)((z + dz + KN) % KN) * KN + (y + dy + KN) % KN) * KN + (x + dx + KN) % KN;
-        if (SPLIT) {
-          f = __half22float2(*reinterpret_cast<const __half2*>(static_cast<const __half*>(a) + q * CP + c));
-          const float2 l = __half22float2(*reinterpret_cast<const __half2*>(static_cast<const __half*>(alo) + q * CP + c));
-          f.x += l.x; f.y += l.y;
-        } else {
-          f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(static_cast<const __nv_bfloat16*>(a) + q * CP + c));
-        }
-      }
-      *reinterpret_cast<float2*>(sa + vv * LA + c) = f;
-    }
-    __syncthreads();
-    for (int vv = grp; vv < VS; vv += NG) {
-      const float4 g0 = *reinterpret_cast<const float4*>(sg + vv * LG + co0);
-      const float4 g1 = *reinterpret_cast<const float4*>(sg + vv * LG + co0 + 4);
-      const float4 aa = *reinterpret_cast<const float4*>(sa + vv * LA + ci0);
-      const float gv[TCO] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-      const float av[TCI] = {aa.x, aa.y, aa.z, aa.w};
-#pragma unroll
-      for (int i = 0; i < TCO; ++i)
-#pragma unroll
-        for (int j = 0; j < TCI; ++j) acc[i][j] = fmaf(gv[i], av[j], acc[i][j]);
-      if (centre) {
-#pragma unroll
-        for (int i = 0; i < TCO; ++i) accb[i] += gv[i];
-      }
-    }
-    __syncthreads();
-  }
-  // the groups' tiles: red[grp][lt][e], e = i TCI + j; entry o = lt NE + e of
-  // a group is (co0(lt) + e / TCI, ci0(lt) + e % TCI)
-  float* red = sbuf;
-#pragma unroll
-  for (int e = 0; e < NE; ++e) red[(grp * TG + lt) * NE + e] = acc[e / TCI][e % TCI];
-  __syncthreads();
-  for (int o = tid; o < TG * NE; o += 256) {
-    float sum = 0.f;
-    for (int k = 0; k < NG; ++k) sum += red[k * TG * NE + o];
-    const int l2 = o / NE, e = o % NE;
-    const int co = TCO * (l2 / (CI / TCI)) + e / TCI, ci = TCI * (l2 % (CI / TCI)) + e % TCI;
-    if (co < cout && ci < cin) atomicAdd(&gw[((long long)co * cin + ci) * 27 + t], double(sum));
-  }
-  if (!centre) return;  // uniform per block
-  __syncthreads();
-  // bias: the threads with ci0 = 0 hold every co once per group
-  if (ci0 == 0) {
-#pragma unroll
-    for (int i = 0; i < TCO; ++i) red[grp * CO + co0 + i] = accb[i];
-  }
-  __syncthreads();
-  if (tid < CO) {
-    float sum = 0.f;
-    for (int k = 0; k < NG; ++k) sum += red[k * CO + tid];
-    if (tid < cout) atomicAdd(&gb[tid], double(sum));
-  }
-}
-
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -858,6 +661,7 @@ template <int KN> static void cnn_init_n() {
 void cnn_init() {
   cnn_init_n<64>();
   cnn_init_n<128>();
+  wgrad_init();
 }
 
 static unsigned nblk(long long n) { return unsigned((n + 255) / 256); }
@@ -925,14 +729,18 @@ void launch_cnn_forward(const CnnArgs& a, cudaStream_t st) {
   else cnn_forward_n<128>(a, st);
 }
 
-// CI, CO: the layer's channels rounded up to the register tile (4 | 32 inputs, 8 | 32 outputs)
-template <int KN, int CP, int COP, int CI, int CO, bool SPLIT = false>
-static void wgrad_launch(const __nv_bfloat16* g, const void* act, int cin, int cout, double* gw, double* gb,
-                         cudaStream_t st, const __nv_bfloat16* glo = nullptr, const void* alo = nullptr) {
-  constexpr long long npts = (long long)KN * KN * KN;
-  const int vchunk = KN >= 128 ? 16384 : 4096;  // 27 x 128 | 27 x 64 blocks: about 6 and 3 full waves
-  dim3 grid(27, unsigned((npts + vchunk - 1) / vchunk));
-  k_conv_wgrad<KN, CP, COP, CI, CO, SPLIT><<<grid, 256, 0, st>>>(g, glo, act, alo, cin, cout, vchunk, gw, gb);
+// weight and bias gradients of layer l from its output gradient (gbf) and its input
+static void wgrad_layer(const CnnBwdArgs& a, int l, cudaStream_t st) {
+  static const int cp[4] = {16, 32, 32, 32}, cop[4] = {32, 32, 32, 16}, cin[4] = {4, 32, 32, 32}, cout[4] = {32, 32, 32, 6};
+  WgradArgs w{};
+  w.g = a.gbf; w.glo = a.gbf_lo;
+  w.a = a.split ? (const void*)a.acth[l] : (const void*)a.act[l];
+  w.alo = a.actl[l];
+  w.cin = cin[l]; w.cout = cout[l];
+  w.gw = a.gw + a.woff[l];
+  w.gb = w.gw + (long long)cout[l] * cin[l] * 27;
+  w.err = a.err; w.nsm = a.nsm; w.wait_limit = a.wait_limit;
+  launch_wgrad(a.n, cp[l], cop[l], a.split, w, st);
 }
 
 template <int KN> static void cnn_backward_n(const CnnBwdArgs& a, cudaStream_t st) {
@@ -940,19 +748,19 @@ template <int KN> static void cnn_backward_n(const CnnBwdArgs& a, cudaStream_t s
   const int grid = a.nsm > 0 ? a.nsm : 148;
   // layer 4: g4 = dL/dtau (BF16 [v][16]); input gradient through W4^T; weight gradient against act3
   k_gtau_cl<<<nblk(npts), 256, 0, st>>>(a.gtau, a.gbf, npts);
-  wgrad_launch<KN, 32, 16, 32, 8>(a.gbf, a.act[3], 32, 6, a.gw + a.woff[3], a.gw + a.woff[3] + 6 * 32 * 27, st);
+  wgrad_layer(a, 3, st);
   ConvOut o{};
   o.pre = a.gf;
   conv_launch<KN, 16, 32, kLinear>(grid, a.gbf, a.wt[3], nullptr, o, a.err, a.wait_limit, st);
   // layers 3, 2: g_pre = g_post * gelu'(h); input and weight gradients
   for (int l = 2; l >= 1; --l) {
     k_gelu_bwd_cl<<<nblk(npts * 32), 256, 0, st>>>(a.gf, a.pre[l], a.gbf, npts * 32);
-    wgrad_launch<KN, 32, 32, 32, 32>(a.gbf, a.act[l], 32, 32, a.gw + a.woff[l], a.gw + a.woff[l] + 32 * 32 * 27, st);
+    wgrad_layer(a, l, st);
     conv_launch<KN, 32, 32, kLinear>(grid, a.gbf, a.wt[l], nullptr, o, a.err, a.wait_limit, st);
   }
   // layer 1: input gradient into 16 channels (4 used), then planar
   k_gelu_bwd_cl<<<nblk(npts * 32), 256, 0, st>>>(a.gf, a.pre[0], a.gbf, npts * 32);
-  wgrad_launch<KN, 16, 32, 4, 32>(a.gbf, a.act[0], 4, 32, a.gw + a.woff[0], a.gw + a.woff[0] + 32 * 4 * 27, st);
+  wgrad_layer(a, 0, st);
   conv_launch<KN, 32, 16, kLinear>(grid, a.gbf, a.wt[0], nullptr, o, a.err, a.wait_limit, st);
   k_gin_planar<<<nblk(npts), 256, 0, st>>>(a.gf, a.gin_planar, npts);
 }
@@ -965,19 +773,16 @@ template <int KN> static void cnn_backward_split_n(const CnnBwdArgs& a, cudaStre
   ConvOut o{};
   o.pre = a.gf;
   k_gtau_cl_split<<<nblk(npts), 256, 0, st>>>(a.gtau, a.gbf, a.gbf_lo, npts);
-  wgrad_launch<KN, 32, 16, 32, 8, true>(a.gbf, a.acth[3], 32, 6, a.gw + a.woff[3], a.gw + a.woff[3] + 6 * 32 * 27, st,
-                                 a.gbf_lo, a.actl[3]);
+  wgrad_layer(a, 3, st);
   conv_split<KN, 16, 32, kAccum, false>(grid, a.gbf, a.gbf_lo, a.wt[3], a.wtl[3], nullptr, o, a.err, a.wait_limit, st);
   for (int l = 2; l >= 1; --l) {
     k_gelu_bwd_cl_split<<<nblk(npts * 32), 256, 0, st>>>(a.gf, a.pre[l], a.gbf, a.gbf_lo, npts * 32);
-    wgrad_launch<KN, 32, 32, 32, 32, true>(a.gbf, a.acth[l], 32, 32, a.gw + a.woff[l], a.gw + a.woff[l] + 32 * 32 * 27, st,
-                                   a.gbf_lo, a.actl[l]);
+    wgrad_layer(a, l, st);
     conv_split<KN, 32, 32, kAccum, false>(grid, a.gbf, a.gbf_lo, a.wt[l], a.wtl[l], nullptr, o, a.err, a.wait_limit,
                                           st);
   }
   k_gelu_bwd_cl_split<<<nblk(npts * 32), 256, 0, st>>>(a.gf, a.pre[0], a.gbf, a.gbf_lo, npts * 32);
-  wgrad_launch<KN, 16, 32, 4, 32, true>(a.gbf, a.acth[0], 4, 32, a.gw + a.woff[0], a.gw + a.woff[0] + 32 * 4 * 27, st,
-                                 a.gbf_lo, a.actl[0]);
+  wgrad_layer(a, 0, st);
   conv_split<KN, 32, 16, kAccum, false>(grid, a.gbf, a.gbf_lo, a.wt[0], a.wtl[0], nullptr, o, a.err, a.wait_limit, st);
   k_gin_planar<<<nblk(npts), 256, 0, st>>>(a.gf, a.gin_planar, npts);
 }
