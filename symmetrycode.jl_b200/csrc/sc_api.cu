@@ -74,6 +74,8 @@ struct sc_plan {
   double* shells = nullptr;  // kc + 3 shell sums of the spectrum and the diagnostics
   int* err = nullptr;       // device word set when a bounded wait of a TMA-fed sweep ran out
   void* fa = nullptr, *fb = nullptr;  // full-spectrum scratch (lazy)
+  void* twr = nullptr;                // twiddle buffer of the filter's reduced grid
+  int nr = 0;                         // its size (0: not filled yet)
   std::vector<void*> allocs;
   cudaStream_t cap = nullptr;
   cudaGraphExec_t g_rk4 = nullptr;
@@ -199,11 +201,15 @@ std::vector<unsigned char> twiddle_image(int n) {
   using C = typename sc::V2<R>::T;
   std::vector<unsigned char> img(sc::twiddle_buffer_bytes(n, sizeof(C)));
   C* h = reinterpret_cast<C*>(img.data());
-  for (int m = 0; m < n; ++m) {
+  for (int m = 0; 2 * m <= n; ++m) {
     const long double pi = 3.141592653589793238462643383279502884L;
     const long double th = 2.0L * pi * (long double)m / (long double)n;
     h[m].x = (R)cosl(th);
     h[m].y = (R)(-sinl(th));
+    if (m > 0) {  // the conjugate half
+      h[n - m].x = h[m].x;
+      h[n - m].y = 2 * m == n ? h[m].y : -h[m].y;
+    }
   }
   if (sc::twiddle_x_offset(n, sizeof(C)) > sizeof(C) * (size_t)n)
     sc::xpair810_twiddles(reinterpret_cast<const float2*>(h), reinterpret_cast<float*>(h + n));
@@ -1020,13 +1026,73 @@ int energy_impl(sc_plan* p, const void* const* u, int compact, int weight_k2, do
   return SC_OK;
 }
 
+// The grid on which the DNS products of the filter are formed.  Only the modes
+// |k_i| <= kout of the products are kept, and the inputs have |k_i| <= kc, so any
+// M > 2 kc + kout points per axis give those modes free of aliasing, as the DNS
+// grid does: 810 -> 640 for 128-point LES data, half the rows and points of every
+// sweep.  Taken when at least a tenth of the points per axis go (256 -> 128 would
+// leave 240: no faster, and a radix-5 size rounds a little more than a power of
+// two).  0: the DNS grid, also where the x sweep does not take the shape.
+int reduced_grid(const sc_plan* p, int kout) {
+  const int m = sc::sweep_size_from(2 * p->kc + kout + 1);
+  return p->D == 3 && m > 0 && 10 * m <= 9 * p->n && p->kc > m / 3 && kout <= m / 5 ? m : 0;
+}
+
+// Fills the plan's second twiddle buffer for size m (once per size).  Not while
+// the stream is being captured: false then, and the caller takes the DNS grid.
+template <typename R>
+bool reduced_twiddles(sc_plan* p, int m, cudaStream_t st) {
+  if (p->nr == m) return true;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
+  if (!sc::init_kernels<R>(m)) return false;
+  const std::vector<unsigned char> img = twiddle_image<R>(m);
+  p->nr = 0;
+  if (cudaMemcpyAsync(p->twr, img.data(), img.size(), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
+    return false;
+  p->nr = m;
+  return true;
+}
+
+// compact u -> F[u_i u_j]/n^D on the compact cube of half-width kout, formed on m points per axis
+template <typename R>
+int products_reduced(sc_plan* p, void* const* u, int kout, int m, void* const* sig, cudaStream_t st) {
+  const int K1 = p->K1, kc = p->kc, K1o = kout + 1, ld = even_up(K1), ldo = even_up(K1o);
+  sc::ColArgs a = z_inverse_args(K1, p->K2, m, kc, ld);
+  for (int c = 0; c < 3; ++c) { a.in[c] = u[c]; a.out[c] = p->be[c]; }
+  a.ncomp = 3;
+  sc::launch_col_inv<R>(m, a, p->twr, st);
+  sc::ColArgs b = y_inverse_args(K1, m, kc, ld);
+  for (int c = 0; c < 3; ++c) { b.in[c] = p->be[c]; b.out[c] = p->cc[c]; }
+  b.ncomp = 3;
+  sc::launch_col_inv<R>(m, b, p->twr, st);
+  sc::XArgs x{};
+  for (int c = 0; c < 3; ++c) x.in[c] = p->cc[c];
+  for (int c = 0; c < 6; ++c) x.out[c] = p->dd[c];
+  x.D = 3; x.K1in = K1; x.K1out = K1o; x.nrows = (long long)m * m; x.scale = 1.0 / ((double)m * m * m);
+  x.ldo = ldo;
+  if (!sc::launch_xsweep_ns<R>(m, x, p->twr, st)) return fail(SC_ERR_SIZE, "no product sweep on %d points", m);
+  sc::ColArgs f = y_forward_args(K1o, m, kout, ldo);
+  for (int c = 0; c < 6; ++c) { f.in[c] = p->dd[c]; f.out[c] = p->be[c]; }
+  f.ncomp = 6;
+  sc::launch_col_fwd<R>(m, f, p->twr, st);
+  sc::ColArgs g = z_forward_args(K1o, m, kout, ldo);
+  for (int c = 0; c < 6; ++c) { g.in[c] = p->be[c]; g.out[c] = sig[c]; }
+  g.ncomp = 6;
+  sc::launch_col_fwd<R>(m, g, p->twr, st);
+  return check_launch("product pipeline");
+}
+
 template <typename R>
 int filter_impl(sc_plan* dns, sc_plan* les, const void* const* u, const double* deltas, int nd,
                 void* const* ubar, void* const* tau, cudaStream_t st) {
   const int D = dns->D;
   int rc = pack_state<R>(dns, u, dns->S, st);
   if (rc) return rc;
-  rc = products<R>(dns, dns->S, st, nullptr, les->kc, dns->sig);
+  const int m = reduced_grid(dns, les->kc);
+  if (m && reduced_twiddles<R>(dns, m, st)) rc = products_reduced<R>(dns, dns->S, les->kc, m, dns->sig, st);
+  else rc = products<R>(dns, dns->S, st, nullptr, les->kc, dns->sig);
   if (rc) return rc;
   for (int d = 0; d < nd; ++d) {
     sc::FilterArgs f{};
@@ -1091,6 +1157,8 @@ int sc_plan_create(sc_plan** out, int D, int n, double l, int dtype, size_t* wor
   bool ok = (dtype == SC_FLOAT64) ? sc::init_kernels<double>(n) : sc::init_kernels<float>(n);
   if (!ok) { rc = fail(SC_ERR_CUDA, "kernel attribute setup failed for n=%d", n); goto bad; }
   if ((rc = plan_alloc(p, &p->tw, sc::twiddle_buffer_bytes(n, p->esz)))) goto bad;
+  // a smaller size's buffer, the pair table of 810 included
+  if (D == 3 && (rc = plan_alloc(p, &p->twr, 3 * (size_t)n * p->esz + sc::xpair810_twiddle_bytes()))) goto bad;
   for (int c = 0; c < D; ++c) {
     if ((rc = plan_alloc(p, &p->U[c], p->csz * p->esz))) goto bad;
     if ((rc = plan_alloc(p, &p->ACC[c], p->csz * p->esz))) goto bad;

@@ -835,7 +835,7 @@ bool launch_xplain_pinned(int N, bool inv, const XPlainArgs& a, const void* tw, 
 }
 
 bool launch_xsweep810(const XArgs& a, const void* tw, cudaStream_t st) {
-  if (a.D != 3 || a.variant == 3) return false;
+  if (a.D != 3 || a.variant == 3 || a.K1in > 271) return false;
   const float2* t2 = static_cast<const float2*>(tw);
   if (a.variant == 1 || a.variant == 2) {
     launch_xpair810(a, t2 + 810, a.variant == 2 ? 4 : 5, st);

@@ -49,4 +49,12 @@ inline bool sweep_size(int n, bool f32, int* xn1 = nullptr, int* xn2 = nullptr) 
   }
 }
 
+// the smallest of these sizes that is at least m (0: none)
+inline int sweep_size_from(int m) {
+#define SC_CASE(N, ...) if (N >= m) return N;
+  SC_SWEEP_SIZES(SC_CASE)
+#undef SC_CASE
+  return 0;
+}
+
 }  // namespace sc

@@ -20,9 +20,11 @@ template <typename R> bool xrow_init(int N) {
 }
 
 // every caller's rows come in pairs (N is even) and indexes fit 32 bits (N <= 1024);
-// inputs of the product sweep and of vmax are compact rows of N / 3 + 1 modes
+// inputs of the product sweep and of vmax are compact rows of N / 3 + 1 modes,
+// or, in 3D with at most N / 5 + 1 modes kept, longer rows of fewer than N / 2 + 1
 template <typename R> bool xrow_ns(int N, const XArgs& a, const void* tw, cudaStream_t st) {
-  if (a.K1in != N / 3 + 1 || a.K1out > a.K1in || (a.nrows & 1)) return false;
+  const bool wide = a.D == 3 && a.K1in > N / 3 + 1 && 2 * (a.K1in - 1) < N && a.K1out <= N / 5 + 1;
+  if ((a.K1in != N / 3 + 1 && !wide) || a.K1out > a.K1in || (a.nrows & 1)) return false;
   switch (N) {
 #define SC_CASE(NN, ...) case NN: XRow<R, NN>::ns(a, xtab<R>(N, tw), st); return true;
     SC_SWEEP_SIZES(SC_CASE)

@@ -118,6 +118,33 @@ __device__ __forceinline__ void xr_i2(const typename V2<R>::T* slot, int i, type
   DFT<Cfg::N2, true, typename V2<R>::T>::run(v);
 }
 
+// I1 with the highest stored mode known at run time only (N / 3 < kmax < N / 2)
+template <typename R, int N>
+__device__ __forceinline__ void xr_i1_wide(const typename V2<R>::T* ra, const typename V2<R>::T* rb, int kmax, bool live,
+                                           int j, const typename V2<R>::T* __restrict__ t1, typename V2<R>::T* slot) {
+  using C = typename V2<R>::T;
+  using Cfg = XRowCfg<R, N>;
+  constexpr int N1 = Cfg::N1, N2 = Cfg::N2;
+  C v[N1];
+#pragma unroll
+  for (int n1 = 0; n1 < N1; ++n1) {
+    const int f = N2 * n1 + j;
+    v[n1] = mk<C>(R(0), R(0));
+    if (!live) continue;
+    const int cls = crange(N2 * n1, N2, N, N / 3 + 1, N / 3);  // 0, 1: stored whatever kmax is
+    if (cls == 0 || (2 * N2 * n1 < N && cls != 1 && f <= kmax)) v[n1] = xr_direct(ra, rb, f, n1 == 0 && j == 0);
+    else if (cls == 1 || (2 * (N2 * n1 + N2) > N && f >= N - kmax)) v[n1] = xr_mirror(ra, rb, N - f);
+  }
+  DFT<N1, true, C>::run(v);
+#pragma unroll
+  for (int k1 = 1; k1 < N1; ++k1) {
+    const C w = __ldg(t1 + k1 * N2 + j);
+    v[k1] = cmul(v[k1], mk<C>(w.x, -w.y));
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < N1; ++k1) slot[k1 * Cfg::SP + j] = v[k1];
+}
+
 // F1 of lane i: v[n] = packed physical values at x = i + N1 n
 template <typename R, int N>
 __device__ __forceinline__ void xr_f1(typename V2<R>::T* v, int i, const typename V2<R>::T* __restrict__ t2,
@@ -160,8 +187,10 @@ template <typename R, int N> __device__ __forceinline__ int xr_at(int k) {
 // r + 1, slot 2 u3(r) + i u3(r + 1); forward, one row at a time, in slots 0, 2,
 // 3: (u1 u1, u2 u2), (u3 u3, u1 u2), (u2 u3, u3 u1).  2D: slots 0, 1 as above;
 // forward (u1 u1, u2 u2) of each row and u1 u2 (r) + i u1 u2 (r + 1).
-// FULL: all N / 3 + 1 modes are kept on the output.
-template <typename R, int N, int D, bool FULL>
+// FULL: all N / 3 + 1 modes are kept on the output.  WIDE: the rows hold up to
+// N / 2 modes (the reduced grid of the DNS -> LES filter) and at most N / 5 + 1
+// are kept, so that most of the last forward radix is never formed.
+template <typename R, int N, int D, bool FULL, bool WIDE = false>
 __global__ void __launch_bounds__(32 * XRowCfg<R, N>::wpc(D == 3 ? 4 : 3),
                                   XRowCfg<R, N>::minb(D == 3 ? 4 : 3, XRowCfg<R, N>::regs_ns))
 k_xr_ns(const __grid_constant__ XArgs a, const typename V2<R>::T* __restrict__ t1, const typename V2<R>::T* __restrict__ t2) {
@@ -170,6 +199,8 @@ k_xr_ns(const __grid_constant__ XArgs a, const typename V2<R>::T* __restrict__ t
   constexpr int N1 = Cfg::N1, N2 = Cfg::N2, W = Cfg::W, PS = Cfg::PS, KC = Cfg::KC;
   constexpr int NI = D == 3 ? 3 : 2;  // inverse pencils of a row pair
   constexpr int WPC = Cfg::wpc(D == 3 ? 4 : 3);
+  constexpr int KO = WIDE ? N / 5 : KC;  // highest mode the forward side may keep
+  const int K1i = WIDE ? a.K1in : KC + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   C* sm = reinterpret_cast<C*>(smem_raw + (threadIdx.x >> 5) * Cfg::slots(D == 3 ? 4 : 3));
@@ -183,9 +214,11 @@ k_xr_ns(const __grid_constant__ XArgs a, const typename V2<R>::T* __restrict__ t
   for (int it = lane; it < W * NI * N2; it += 32) {
     const int w = it / (NI * N2), p = (it / N2) % NI, j = it % N2;
     const int row = 2 * (rp0 + w);
-    const C* ra = (p < 2 ? in0 : in2) + (row + (p == 1)) * (KC + 1);
-    const C* rb = p < 2 ? in1 + (row + p) * (KC + 1) : in2 + (row + 1) * (KC + 1);
-    xr_i1<R, N, KC>(ra, rb, rp0 + w < npair, j, t1, sm + (p * W + w) * PS);
+    const C* ra = (p < 2 ? in0 : in2) + (row + (p == 1)) * K1i;
+    const C* rb = p < 2 ? in1 + (row + p) * K1i : in2 + (row + 1) * K1i;
+    C* slot = sm + (p * W + w) * PS;
+    if constexpr (WIDE) xr_i1_wide<R, N>(ra, rb, K1i - 1, rp0 + w < npair, j, t1, slot);
+    else xr_i1<R, N, KC>(ra, rb, rp0 + w < npair, j, t1, slot);
   }
   __syncwarp();
   const int w = lane / N1, i = lane - w * N1;
@@ -222,7 +255,7 @@ k_xr_ns(const __grid_constant__ XArgs a, const typename V2<R>::T* __restrict__ t
           xr_f1<R, N>(v, i, t2, sm + (3 * W + w) * PS);
         }
         __syncwarp();
-        for (int it = lane; it < W * N2; it += 32) xr_f2<R, N, KC>(sm + (3 * W + it / N2) * PS, it % N2);
+        for (int it = lane; it < W * N2; it += 32) xr_f2<R, N, KO>(sm + (3 * W + it / N2) * PS, it % N2);
         __syncwarp();
         for (int it = lane; it < W * K1o; it += 32) {
           const int ww = it / K1o, kx = it - ww * K1o;
@@ -272,7 +305,7 @@ k_xr_ns(const __grid_constant__ XArgs a, const typename V2<R>::T* __restrict__ t
       for (int it = lane; it < W * 3 * N2; it += 32) {
         const int q = it / N2, kp = it - q * N2;  // slot 0, 2, 3 of row pair q % W
         const int b = q / W;
-        xr_f2<R, N, KC>(sm + ((b ? b + 1 : 0) * W + q - b * W) * PS, kp);
+        xr_f2<R, N, KO>(sm + ((b ? b + 1 : 0) * W + q - b * W) * PS, kp);
       }
       __syncwarp();
       for (int it = lane; it < W * K1o; it += 32) {
@@ -488,6 +521,7 @@ template <typename R, int N> void XRow<R, N>::init() {
   constexpr size_t s3 = Cfg::wpc(3) * Cfg::slots(3), s4 = Cfg::wpc(4) * Cfg::slots(4);
   xr_smem(k_xr_ns<R, N, 3, true>, s4);
   xr_smem(k_xr_ns<R, N, 3, false>, s4);
+  xr_smem(k_xr_ns<R, N, 3, false, true>, s4);
   xr_smem(k_xr_ns<R, N, 2, true>, s3);
   xr_smem(k_xr_ns<R, N, 2, false>, s3);
   xr_smem(k_xr_c2r<R, N, N / 3>, s3);
@@ -517,7 +551,8 @@ template <typename R, int N> void XRow<R, N>::ns(const XArgs& a, const void* tx,
   }
   constexpr int wpc = Cfg::wpc(4);
   const unsigned nb = xr_grid(a.nrows / 2, Cfg::W, wpc);
-  if (a.K1out == N / 3 + 1) k_xr_ns<R, N, 3, true><<<nb, 32 * wpc, wpc * Cfg::slots(4), st>>>(a, t1, t2);
+  if (a.K1in != N / 3 + 1) k_xr_ns<R, N, 3, false, true><<<nb, 32 * wpc, wpc * Cfg::slots(4), st>>>(a, t1, t2);
+  else if (a.K1out == N / 3 + 1) k_xr_ns<R, N, 3, true><<<nb, 32 * wpc, wpc * Cfg::slots(4), st>>>(a, t1, t2);
   else k_xr_ns<R, N, 3, false><<<nb, 32 * wpc, wpc * Cfg::slots(4), st>>>(a, t1, t2);
 }
 

@@ -88,3 +88,32 @@ def test_3d_product_sweep_matches_triad_sums(n, dtype):
         num += float(torch.linalg.vector_norm(du[c]).double() ** 2)
     assert math.sqrt(num / den) < (1e-12 if dtype == torch.float64 else 1e-5)
     g.close()
+
+
+@pytest.mark.parametrize("captured", (False, True))
+@pytest.mark.parametrize("n,m", ((96, 36), (60, 20), (120, 36), (160, 64), (192, 32)))
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_sfs_on_the_reduced_grid_matches_the_oracle(n, m, dtype, captured):
+    """DNS products formed on fewer points than the DNS grid has (96 -> 80, 60 ->
+    48, 120 -> 96, 160 -> 128, 192 -> 160), and on the DNS grid where the first
+    call is being captured.  Tolerances as in test_gpu_filter.py: tau against the
+    size of the products it cancels."""
+    gd, gl = (S.Grid(3, k, dtype=dtype, device="cuda:0") for k in (n, m))
+    od, ol = O.Grid(3, n), O.Grid(3, m)
+    u = O.random_field(od, seed=5, kpeak=4)
+    d = 2 * ol.l / m
+    ud = [to_dev(c, gd) for c in u]
+    ub, tau = S.vectorfield(gl), S.tensorfield(gl)
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            S.sfs_(ub, tau, ud, gd, gl, d)
+        graph.replay()
+    else:
+        S.sfs_(ub, tau, ud, gd, gl, d)
+    rb, rt = O.sfs(u, od, ol, d)
+    tol = 1e-12 if dtype == torch.float64 else 1e-5
+    assert rel_l2([to_np(c) for c in ub], rb) < tol
+    s1 = [O.twothirds(O.gaussianfilter(O.cutoff(c, od, ol), d, ol), ol) for c in O.nonlinearity(u, od)]
+    scale = math.sqrt(sum(float(np.sum(np.abs(c) ** 2)) for c in s1))
+    assert math.sqrt(sum(float(np.sum(np.abs(to_np(x) - y) ** 2)) for x, y in zip(tau, rt))) < tol * scale
