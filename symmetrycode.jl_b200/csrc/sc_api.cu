@@ -107,6 +107,7 @@ struct sc_closure {
   void* ph4[3] = {};  // physical test-filtered velocity
   void* bb[12] = {};  // batched-transform scratch (kx, ky, z), stored [ky][z][kx]
   void* cb[12] = {};  // batched-transform scratch (kx, y, z)
+  void* wtab = nullptr;    // test filter's Gaussian by |k|^2 (Bardina, dynamic Smagorinsky; sizes with register sweeps)
   double* dsum = nullptr;  // [<ML>, <MM>, c] (dynamic Smagorinsky); [a2, -, -, z] (CNN)
   // CNN closure
   void* cw[4] = {};   // packed BF16 weights per layer
@@ -369,7 +370,7 @@ int products(sc_plan* p, void* const* u, cudaStream_t st, cudaEvent_t* ev = null
 // ---------------------------------------------------------------------------
 template <typename R>
 int c2p_batch(sc_plan* p, void* const* bb, void* const* cb, void* const* in, void* const* out, int m,
-              cudaStream_t st, bool pinned = false) {
+              cudaStream_t st, bool pinned = false, const void* wtab = nullptr) {
   const int n = p->n, K1 = p->K1, K2 = p->K2, kc = p->kc;
   for (int c0 = 0; c0 < m; c0 += 12) {
     const int mc = m - c0 < 12 ? m - c0 : 12;
@@ -377,7 +378,7 @@ int c2p_batch(sc_plan* p, void* const* bb, void* const* cb, void* const* in, voi
     if (p->D == 3) {
       a = z_inverse_args(K1, K2, n, kc);
       for (int c = 0; c < mc; ++c) { a.in[c] = in[c0 + c]; a.out[c] = bb[c]; }
-      a.ncomp = mc;
+      a.ncomp = mc; a.wtab = wtab;
       sc::launch_col_inv<R>(n, a, p->tw, st);
       sc::ColArgs b = y_inverse_args(K1, n, kc);
       for (int c = 0; c < mc; ++c) { b.in[c] = bb[c]; b.out[c] = cb[c]; }
@@ -385,7 +386,7 @@ int c2p_batch(sc_plan* p, void* const* bb, void* const* cb, void* const* in, voi
       sc::launch_col_inv<R>(n, b, p->tw, st);
     } else {
       for (int c = 0; c < mc; ++c) { a.in[c] = in[c0 + c]; a.out[c] = cb[c]; }
-      a.ncomp = mc; a.K1 = K1; a.ncols = 1;
+      a.ncomp = mc; a.K1 = K1; a.ncols = 1; a.wtab = wtab;
       a.in_cs = 0; a.in_es = K1; a.out_cs = 0; a.out_es = K1;
       a.kpos = kc + 1; a.kneg = kc; a.zero_origin = 1;
       sc::launch_col_inv<R>(n, a, p->tw, st);
@@ -524,6 +525,42 @@ int cc_backward(sc_closure* cl, const R* gtau, cudaStream_t st) {
   return check_launch("cnn backward (CUDA cores)");
 }
 
+// Compact fields -> the closure's point function in physical space -> compact
+// stress in cl->th, the three x passes in one sweep (sc::launch_x_point);
+// *done = false where the size or dimension has no such sweep.  Scratch: bb, cb, tp.
+template <typename R>
+int point_batch(sc_closure* cl, void* const* in, int nin, int kind, double delta, double p0, bool* done,
+                cudaStream_t st) {
+  sc_plan* p = cl->p;
+  const int n = p->n, K1 = p->K1, kc = p->kc;
+  *done = false;
+  if (p->D != 3 || !sc::sweep_size(n, p->dtype == SC_FLOAT32)) return SC_OK;
+  sc::ColArgs a = z_inverse_args(K1, p->K2, n, kc);
+  for (int c = 0; c < nin; ++c) { a.in[c] = in[c]; a.out[c] = cl->bb[c]; }
+  a.ncomp = nin;
+  sc::launch_col_inv<R>(n, a, p->tw, st);
+  sc::ColArgs b = y_inverse_args(K1, n, kc);
+  for (int c = 0; c < nin; ++c) { b.in[c] = cl->bb[c]; b.out[c] = cl->cb[c]; }
+  b.ncomp = nin;
+  sc::launch_col_inv<R>(n, b, p->tw, st);
+  sc::XPointArgs x{};
+  for (int c = 0; c < nin; ++c) x.in[c] = cl->cb[c];
+  for (int c = 0; c < 6; ++c) x.out[c] = cl->tp[c];  // n^3 reals hold n^2 (n / 3 + 1) complex modes
+  x.nin = nin; x.kind = kind; x.delta = delta; x.p0 = p0;
+  x.nrows = (long long)n * n; x.scale = 1.0 / std::pow((double)n, 3);
+  if (!sc::launch_x_point<R>(n, x, p->tw, st)) return fail(SC_ERR_SIZE, "no closure sweep for n=%d", n);
+  sc::ColArgs f = y_forward_args(K1, n, kc);
+  for (int c = 0; c < 6; ++c) { f.in[c] = cl->tp[c]; f.out[c] = cl->bb[c]; }
+  f.ncomp = 6;
+  sc::launch_col_fwd<R>(n, f, p->tw, st);
+  sc::ColArgs g = z_forward_args(K1, n, kc);
+  for (int c = 0; c < 6; ++c) { g.in[c] = cl->bb[c]; g.out[c] = cl->th[c]; }
+  g.ncomp = 6;
+  sc::launch_col_fwd<R>(n, g, p->tw, st);
+  *done = true;
+  return check_launch("closure sweep");
+}
+
 sc::MlpArgs mlp_args(sc_closure* cl, const void* const* G, void* const* tau) {
   sc_plan* p = cl->p;
   sc::MlpArgs a{};
@@ -625,6 +662,21 @@ int tc_backward(sc_closure* cl, cudaStream_t st) {
   return check_launch("cnn backward (tensor cores)");
 }
 
+// Test-filtered compact fields (width `delta`) in physical space.  The sweeps
+// multiply by the closure's table while they gather; elsewhere a pass over the
+// modes writes the filtered fields to `tmp` first (may be `in`).
+template <typename R>
+int filtered_to_phys(sc_closure* cl, void* const* in, void* const* tmp, void* const* out, int m, double delta,
+                     cudaStream_t st) {
+  sc_plan* p = cl->p;
+  if (cl->wtab) return c2p_batch<R>(p, cl->bb, cl->cb, in, out, m, st, false, cl->wtab);
+  sc::LesSpecArgs f = spec_args(p);
+  for (int c = 0; c < m; ++c) { f.in[c] = in[c]; f.out[c] = tmp[c]; }
+  f.ncomp = m; f.delta = delta;
+  sc::launch_spec_filter<R>(f, p->D, st);
+  return c2p_batch<R>(p, cl->bb, cl->cb, tmp, out, m, st);
+}
+
 // Closure stress of the compact state u into cl->th (compact), i.e. the
 // spectrum to_spec!(model(u, G)) that les! adds to sigma (src/les.jl:19-27).
 // Bardina and dynamic Smagorinsky read the product spectra F[u_i u_j]/n^D from
@@ -647,6 +699,10 @@ int closure_tauhat(sc_closure* cl, void* const* u, cudaStream_t st, void* const*
     for (int c = 0; c < D; ++c) g.in[c] = u[c];
     for (int c = 0; c < D * D; ++c) g.out[c] = cl->gc[c];
     sc::launch_grad<R>(g, D, st);
+    bool done = false;
+    if (!tau_phys_out &&
+        ((rc = point_batch<R>(cl, cl->gc, 9, cl->kind, cl->delta, cl->prm[0], &done, st)) || done))
+      return rc;
     if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, cl->gc, cl->gp, D * D, st))) return rc;
     sc::LesPhysArgs a = phys_args(p);
     for (int c = 0; c < D * D; ++c) a.in[c] = cl->gp[c];
@@ -654,17 +710,8 @@ int closure_tauhat(sc_closure* cl, void* const* u, cudaStream_t st, void* const*
     a.kind = cl->kind; a.delta = cl->delta; a.p0 = cl->prm[0];
     sc::launch_closure_pt<R>(a, D, st);
   } else if (cl->kind == sc::kBardina) {
-    const double dt_ = cl->prm[0] * cl->delta;
-    sc::LesSpecArgs f = spec_args(p);
-    for (int c = 0; c < D; ++c) { f.in[c] = u[c]; f.out[c] = cl->ut[c]; }
-    f.ncomp = D; f.delta = dt_;
-    sc::launch_spec_filter<R>(f, D, st);
-    sc::LesSpecArgs h = spec_args(p);
-    for (int c = 0; c < NP; ++c) { h.in[c] = p->sig[c]; h.out[c] = cl->gc[c]; }
-    h.ncomp = NP; h.delta = dt_;
-    sc::launch_spec_filter<R>(h, D, st);
-    if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, cl->gc, cl->gp, NP, st))) return rc;
-    if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, cl->ut, cl->ph4, D, st))) return rc;
+    if ((rc = filtered_to_phys<R>(cl, p->sig, cl->gc, cl->gp, NP, cl->prm[0] * cl->delta, st))) return rc;
+    if ((rc = filtered_to_phys<R>(cl, u, cl->ut, cl->ph4, D, cl->prm[0] * cl->delta, st))) return rc;
     sc::LesPhysArgs a = phys_args(p);
     for (int c = 0; c < NP; ++c) { a.in[c] = cl->gp[c]; a.out[c] = cl->tp[c]; }
     for (int c = 0; c < D; ++c) a.in2[c] = cl->ph4[c];
@@ -672,44 +719,29 @@ int closure_tauhat(sc_closure* cl, void* const* u, cudaStream_t st, void* const*
     sc::launch_sub_products<R>(a, D, st);
   } else if (cl->kind == sc::kDynSmagorinsky) {
     const double dtl = 2.0 * cl->delta, ddb = std::sqrt(dtl * dtl + cl->delta * cl->delta);
-    sc::LesSpecArgs f = spec_args(p);  // u~ = P G~ u
-    for (int c = 0; c < D; ++c) { f.in[c] = u[c]; f.out[c] = cl->ut[c]; }
-    f.ncomp = D; f.delta = dtl;
-    sc::launch_spec_filter<R>(f, D, st);
-    sc::LesSpecArgs h = spec_args(p);  // P G~ sigma
-    for (int c = 0; c < NP; ++c) { h.in[c] = p->sig[c]; h.out[c] = cl->gc[c]; }
-    h.ncomp = NP; h.delta = dtl;
-    sc::launch_spec_filter<R>(h, D, st);
     sc::LesSpecArgs sr = spec_args(p);  // S-hat
     for (int c = 0; c < D; ++c) sr.in[c] = u[c];
     for (int c = 0; c < NP; ++c) sr.out[c] = cl->s2[c];
     sc::launch_strain<R>(sr, D, st);
-    if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, cl->gc, cl->gp, NP, st))) return rc;   // L1
-    if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, cl->ut, cl->ph4, D, st))) return rc;   // u~
-    if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, cl->s2, cl->tp, NP, st))) return rc;   // S
-    sc::LesSpecArgs h2 = spec_args(p);  // P G~ P S-hat, in place
-    for (int c = 0; c < NP; ++c) { h2.in[c] = cl->s2[c]; h2.out[c] = cl->s2[c]; }
-    h2.ncomp = NP; h2.delta = dtl;
-    sc::launch_spec_filter<R>(h2, D, st);
-    if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, cl->s2, cl->ph3, NP, st))) return rc;  // S~
-    sc::LesPhysArgs m1 = phys_args(p);  // m1 = smag(S, Delta), in place
-    for (int c = 0; c < NP; ++c) { m1.in[c] = cl->tp[c]; m1.out[c] = cl->tp[c]; }
-    m1.delta = cl->delta;
-    sc::launch_smag_tensor<R>(m1, D, st);
-    sc::LesPhysArgs m2 = phys_args(p);  // m2 = smag(S~, sqrt(5) Delta), in place
-    for (int c = 0; c < NP; ++c) { m2.in[c] = cl->ph3[c]; m2.out[c] = cl->ph3[c]; }
-    m2.delta = ddb;
-    sc::launch_smag_tensor<R>(m2, D, st);
-    if ((rc = p2c_batch<R>(p, cl->bb, cl->cb, cl->tp, cl->th, NP, st))) return rc;   // F[m1]
-    sc::LesSpecArgs h3 = spec_args(p);  // P G~ F[m1]
-    for (int c = 0; c < NP; ++c) { h3.in[c] = cl->th[c]; h3.out[c] = cl->s2[c]; }
-    h3.ncomp = NP; h3.delta = dtl;
-    sc::launch_spec_filter<R>(h3, D, st);
-    if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, cl->s2, cl->ph2, NP, st))) return rc;  // M1
+    if ((rc = filtered_to_phys<R>(cl, p->sig, cl->gc, cl->gp, NP, dtl, st))) return rc;  // L1 = P G~ sigma
+    if ((rc = filtered_to_phys<R>(cl, u, cl->ut, cl->ph4, D, dtl, st))) return rc;       // u~ = P G~ u
+    bool done = false;  // F[m1], m1 = smag(S, Delta)
+    if ((rc = point_batch<R>(cl, cl->s2, 6, 0, cl->delta, 0.0, &done, st))) return rc;
+    if (!done) {
+      if ((rc = c2p_batch<R>(p, cl->bb, cl->cb, cl->s2, cl->tp, NP, st))) return rc;     // S
+      sc::LesPhysArgs m1 = phys_args(p);
+      for (int c = 0; c < NP; ++c) { m1.in[c] = cl->tp[c]; m1.out[c] = cl->tp[c]; }
+      m1.delta = cl->delta;
+      sc::launch_smag_tensor<R>(m1, D, st);
+      if ((rc = p2c_batch<R>(p, cl->bb, cl->cb, cl->tp, cl->th, NP, st))) return rc;
+    }
+    if ((rc = filtered_to_phys<R>(cl, cl->s2, cl->s2, cl->ph3, NP, dtl, st))) return rc;  // S~ = P G~ P S
+    if ((rc = filtered_to_phys<R>(cl, cl->th, cl->s2, cl->ph2, NP, dtl, st))) return rc;  // M1 = P G~ F[m1]
     SC_CU(cudaMemsetAsync(cl->dsum, 0, 3 * sizeof(double), st));
     sc::LesPhysArgs ml = phys_args(p);
     for (int c = 0; c < NP; ++c) { ml.in[c] = cl->gp[c]; ml.in3[c] = cl->ph2[c]; ml.in4[c] = cl->ph3[c]; }
     for (int c = 0; c < D; ++c) ml.in2[c] = cl->ph4[c];
+    ml.delta = ddb;  // m2 = smag(S~, sqrt(5) Delta) is formed there
     sc::launch_dynsmag_mlmm<R>(ml, D, cl->dsum, st);
     sc::LesSpecArgs sc_ = spec_args(p);  // tau-hat = c P F[m1]
     for (int c = 0; c < NP; ++c) { sc_.in[c] = cl->th[c]; sc_.out[c] = cl->th[c]; }
@@ -1539,6 +1571,18 @@ int sc_closure_create(sc_closure** out, sc_plan* p, int kind, double delta, cons
     for (int c = 0; c < 12 && !rc; ++c) rc = A(&cl->cb[c], plane);
     for (int c = 0; c < 12 && !rc && D == 3; ++c) rc = A(&cl->bb[c], mid);
     if (!rc) rc = A((void**)&cl->dsum, 4 * sizeof(double));
+    // Bardina and dynamic Smagorinsky filter at one width only: its Gaussian at
+    // every |k|^2 of the cube, read by the inverse z sweeps (y in 2D)
+    if (!rc && (kind == sc::kBardina || kind == sc::kDynSmagorinsky) && sc::sweep_size(p->n, p->dtype == SC_FLOAT32)) {
+      const int nq = D * p->kc * p->kc + 1;
+      const double width = kind == sc::kBardina ? cl->prm[0] * delta : 2.0 * delta, kfac = 2.0 * M_PI / p->l;
+      rc = A(&cl->wtab, nq * (p->esz / 2));
+      if (!rc) {
+        if (p->dtype == SC_FLOAT64) sc::launch_gauss_table<double>(cl->wtab, nq, kfac, width, 0);
+        else sc::launch_gauss_table<float>(cl->wtab, nq, kfac, width, 0);
+        if (cudaStreamSynchronize(0) != cudaSuccess) rc = fail(SC_ERR_CUDA, "test filter table");
+      }
+    }
   }
   if (rc) {
     for (void* a : cl->allocs) cudaFree(a);

@@ -41,7 +41,8 @@ template <typename R, int N, int T, int S = 0> struct Col2Cfg {
 // or N2 stores (forward) touch a retained mode is known at compile time except
 // in the one block that straddles a boundary; the unused forward outputs are
 // then never formed.
-template <typename R, int N, int T, bool INV, bool FULL, int S = 0>
+// FILT: the gather multiplies by ColArgs::wtab (a closure's test filter).
+template <typename R, int N, int T, bool INV, bool FULL, int S = 0, bool FILT = false>
 __global__ void __launch_bounds__(Col2Cfg<R, N, T, S>::NT, Col2Cfg<R, N, T, S>::MINB)
 k_col2(const __grid_constant__ ColArgs a, const typename V2<R>::T* __restrict__ tw) {
   using C = typename V2<R>::T;
@@ -72,7 +73,14 @@ k_col2(const __grid_constant__ ColArgs a, const typename V2<R>::T* __restrict__ 
         const int rg = FULL ? crange(N2 * n1, N2, N, KP, KN) : 3;
         if (rg == 2) continue;
         const int p = rg == 0 ? e : (rg == 1 ? e - N + Kc : cpos(e, N, kpos, kneg));
-        if (live && p >= 0 && !(a.zero_origin && kx == 0 && c == 0 && p == 0)) v[n1] = __ldg(base + p * ies);
+        if (live && p >= 0 && !(a.zero_origin && kx == 0 && c == 0 && p == 0)) {
+          v[n1] = __ldg(base + p * ies);
+          if constexpr (FILT) {
+            const int ke = p < kpos ? p : p - Kc, kc = c < kpos ? c : c - Kc;
+            const R w = __ldg(static_cast<const R*>(a.wtab) + kx * kx + kc * kc + ke * ke);
+            v[n1] = mk<C>(w * v[n1].x, w * v[n1].y);
+          }
+        }
       }
     } else {
       const C* bj = base + j * ies;
@@ -140,6 +148,7 @@ template <typename R, int N> void ColSweep<R, N>::init() {
     cudaFuncSetAttribute(k_col2<R, N, T, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b));
     cudaFuncSetAttribute(k_col2<R, N, T, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b));
     cudaFuncSetAttribute(k_col2<R, N, T, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b));
+    cudaFuncSetAttribute(k_col2<R, N, T, true, true, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b));
   }
 }
 
@@ -150,7 +159,8 @@ template <typename R, int N> void ColSweep<R, N>::launch(bool inv, const ColArgs
   const dim3 grid((a.K1 + T - 1) / T, a.ncols, a.ncomp);
   const C* t2 = static_cast<const C*>(tw);
   const bool full = a.kpos == N / 3 + 1 && a.kneg == N / 3;
-  if (inv && full) k_col2<R, N, T, true, true><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
+  if (inv && full && a.wtab) k_col2<R, N, T, true, true, 0, true><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
+  else if (inv && full) k_col2<R, N, T, true, true><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
   else if (inv) k_col2<R, N, T, true, false><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
   else if (full) k_col2<R, N, T, false, true><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);
   else k_col2<R, N, T, false, false><<<grid, Cfg::NT, Cfg::SMEM, st>>>(a, t2);

@@ -23,6 +23,9 @@ struct ColArgs {
   long long in_cs, in_es, out_cs, out_es;
   int kpos, kneg;     // compact mapping of the transform axis
   int zero_origin;    // inverse only: treat (kx, c, e) = (0, 0, 0) as zero (k = 0 mode)
+  // inverse, solver layout (kpos = n/3 + 1, kneg = n/3), columns c = ky of the
+  // compact cube: each mode times wtab[kx^2 + ky^2 + e^2] (nullptr: none)
+  const void* wtab;
   int variant;  // FP32 fast sizes: kernel variant chosen by the autotuner (0 = default)
   // bounded device waits of the TMA-fed sweeps: polls before a wait gives up
   // and the plan's device error word it then sets (nullptr: no TMA sweep)
@@ -54,6 +57,18 @@ struct XPlainArgs {
   long long nrows;
   double scale;    // applied to the output
   bool pinned;     // FP32 n = 64, 128: the kernels of the one-pass BF16 network (launch_xplain_pinned)
+};
+
+// Fused x sweep of a closure: c2r of `nin` compact fields, the closure's point
+// function, r2c of the six stress components, times `scale`.
+struct XPointArgs {
+  const void* in[9];
+  void* out[6];
+  int nin;         // 6: strain rate -> its Smagorinsky tensor; 9: velocity gradient -> `kind`
+  int kind;        // nin = 9: kClark, kSmagorinsky, kVerstappen (sc_les.h)
+  double delta, p0;
+  long long nrows;
+  double scale;
 };
 
 // Pointwise spectral epilogue over the compact 2/3 cube (see k_epilogue).
@@ -106,6 +121,8 @@ template <typename R> bool launch_col_inv(int N, const ColArgs& a, const void* t
 template <typename R> bool launch_col_fwd(int N, const ColArgs& a, const void* tw, cudaStream_t st);
 template <typename R> bool launch_xsweep_ns(int N, const XArgs& a, const void* tw, cudaStream_t st);
 template <typename R> bool launch_x_c2r(int N, const XPlainArgs& a, const void* tw, cudaStream_t st);
+// 3D only; false: the size has no fused sweep
+template <typename R> bool launch_x_point(int N, const XPointArgs& a, const void* tw, cudaStream_t st);
 template <typename R> bool launch_x_r2c(int N, const XPlainArgs& a, const void* tw, cudaStream_t st);
 template <typename R> void launch_epilogue(const EpiArgs& a, cudaStream_t st);
 template <typename R> void launch_filter(const FilterArgs& a, cudaStream_t st);

@@ -869,7 +869,7 @@ template <typename R> static bool use_fast(int N) {
 }
 
 template <typename R> bool launch_col_inv(int N, const ColArgs& a, const void* tw, cudaStream_t st) {
-  if (use_fast<R>(N)) return launch_col2(N, true, a, tw, st);
+  if (use_fast<R>(N) && !a.wtab) return launch_col2(N, true, a, tw, st);
   if (col_sweep<R>(N, true, a, tw, st)) return true;
   switch (N) {
 #define SC_CASE(NN) case NN: return col_inv_n<R, NN>(a, tw, st);
@@ -908,6 +908,9 @@ template <typename R> bool launch_x_c2r(int N, const XPlainArgs& a, const void* 
 #undef SC_CASE
     default: return false;
   }
+}
+template <typename R> bool launch_x_point(int N, const XPointArgs& a, const void* tw, cudaStream_t st) {
+  return xrow_point<R>(N, a, tw, st);
 }
 template <typename R> bool launch_x_r2c(int N, const XPlainArgs& a, const void* tw, cudaStream_t st) {
   if (sizeof(R) == 4 && a.pinned && launch_xplain_pinned(N, false, a, tw, st)) return true;
@@ -1074,6 +1077,7 @@ template <typename R> void launch_project_full(const PackArgs& a, double kfac, c
   template bool launch_col_fwd<R>(int, const ColArgs&, const void*, cudaStream_t);                      \
   template bool launch_xsweep_ns<R>(int, const XArgs&, const void*, cudaStream_t);                      \
   template bool launch_x_c2r<R>(int, const XPlainArgs&, const void*, cudaStream_t);                     \
+  template bool launch_x_point<R>(int, const XPointArgs&, const void*, cudaStream_t);                    \
   template bool launch_x_r2c<R>(int, const XPlainArgs&, const void*, cudaStream_t);                     \
   template void launch_epilogue<R>(const EpiArgs&, cudaStream_t);                                       \
   template void launch_pack<R>(const PackArgs&, cudaStream_t);                                          \

@@ -8,6 +8,7 @@
 #include <math.h>
 
 #include "sc_fft.cuh"
+#include "sc_closure_pt.cuh"
 #include "sc_les.h"
 
 namespace sc {
@@ -94,6 +95,13 @@ __global__ void k_spec_filter(const LesSpecArgs a) {
   }
 }
 
+// the same Gaussian by |k|^2 in units of (2 pi / l)^2: w[q], q = 0 .. n - 1
+template <typename R> __global__ void k_gauss_table(R* w, int n, double kfac, double delta) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  w[q] = R(delta > 0 && q >= 9 ? exp(-delta * delta * (kfac * kfac * double(q)) / 24.0) : 1.0);
+}
+
 // ---------------------------------------------------------------------------
 // physical pointwise kernels
 // ---------------------------------------------------------------------------
@@ -124,46 +132,7 @@ __global__ void k_closure_pt(const LesPhysArgs a) {
   R G[3][3] = {};
   load_grad<R, D>(a, i, G);
   R t[3][3] = {};
-  const R d2 = R(a.delta * a.delta);
-  if (a.kind == kClark) {
-    for (int p = 0; p < D; ++p)
-      for (int q = 0; q < D; ++q) {
-        R s = 0;
-        for (int k = 0; k < D; ++k) s += G[p][k] * G[q][k];
-        t[p][q] = d2 / R(12) * s;
-      }
-  } else {
-    R S[3][3];
-    R ss = 0;
-    for (int p = 0; p < D; ++p)
-      for (int q = 0; q < D; ++q) {
-        S[p][q] = (G[p][q] + G[q][p]) / R(2);
-        ss += S[p][q] * S[p][q];
-      }
-    R nu;
-    if (a.kind == kSmagorinsky) {
-      const R cs = R(a.p0);
-      nu = cs * cs * d2 * sqrt(R(2) * ss);
-    } else {  // Verstappen: q = tr(S S)/2, r = tr(S S S)/3, nu = C^2 Delta^2 |r| / q
-      R SS[3][3];
-      for (int p = 0; p < 3; ++p)
-        for (int q = 0; q < 3; ++q) {
-          R s = 0;
-          for (int k = 0; k < 3; ++k) s += S[p][k] * S[k][q];
-          SS[p][q] = s;
-        }
-      R trss = 0, trsss = 0;
-      for (int p = 0; p < 3; ++p) {
-        trss += SS[p][p];
-        for (int k = 0; k < 3; ++k) trsss += SS[p][k] * S[k][p];
-      }
-      const R qq = trss / R(2), rr = trsss / R(3);
-      const R c = R(a.p0);
-      nu = c * c * d2 * fabs(rr) / qq;
-    }
-    for (int p = 0; p < D; ++p)
-      for (int q = 0; q < D; ++q) t[p][q] = -R(2) * nu * S[p][q];
-  }
+  closure_point<R, D>(a.kind, R(a.delta * a.delta), R(a.p0), G, t);
   store_sym<R, D>(a, i, t);
 }
 
@@ -175,10 +144,7 @@ __global__ void k_smag_tensor(const LesPhysArgs a) {
   constexpr int NP = D == 3 ? 6 : 3;
   R s[6];
   for (int q = 0; q < NP; ++q) s[q] = static_cast<const R*>(a.in[q])[i];
-  R s2 = 0;
-  for (int q = 0; q < D; ++q) s2 += s[q] * s[q];
-  for (int q = D; q < NP; ++q) s2 += R(2) * s[q] * s[q];
-  const R nu = R(a.delta * a.delta) * sqrt(R(2) * s2);
+  const R nu = smag_viscosity<R, D>(R(a.delta * a.delta), s);
   for (int q = 0; q < NP; ++q) static_cast<R*>(a.out[q])[i] = -R(2) * nu * s[q];
 }
 
@@ -222,7 +188,8 @@ __device__ __forceinline__ double block_sum_d(double v) {
   return v;
 }
 
-// smagorinsky_ml_mm! (src/closures.jl:152-179) on L = L1 - u~_i u~_j, M = M1 - m2,
+// smagorinsky_ml_mm! (src/closures.jl:152-179) on L = L1 - u~_i u~_j, M = M1 - m2
+// with m2 = smagorinsky_tensor!(S~) formed here from S~ (in4),
 // summed in FP64: sums[0] += sum(M:L), sums[1] += sum(M:M)
 template <typename R, int D>
 __global__ void k_dynsmag_mlmm(const LesPhysArgs a, double* sums) {
@@ -234,11 +201,13 @@ __global__ void k_dynsmag_mlmm(const LesPhysArgs a, double* sums) {
        i += (long long)gridDim.x * blockDim.x) {
     R u[3];
     for (int c = 0; c < D; ++c) u[c] = static_cast<const R*>(a.in2[c])[i];
-    R L[6], M[6];
+    R L[6], M[6], s[6];
+    for (int q = 0; q < NP; ++q) s[q] = static_cast<const R*>(a.in4[q])[i];
+    const R nu = smag_viscosity<R, D>(R(a.delta * a.delta), s);
     for (int q = 0; q < NP; ++q) {
       const int ii = D == 3 ? PI3[q] : PI2[q], jj = D == 3 ? PJ3[q] : PJ2[q];
       L[q] = static_cast<const R*>(a.in[q])[i] - u[ii] * u[jj];
-      M[q] = static_cast<const R*>(a.in3[q])[i] - static_cast<const R*>(a.in4[q])[i];
+      M[q] = static_cast<const R*>(a.in3[q])[i] - (-R(2) * nu * s[q]);
     }
     R tr = 0;
     for (int q = 0; q < D; ++q) tr += L[q];
@@ -281,6 +250,9 @@ template <typename R> void launch_spec_filter(const LesSpecArgs& a, int D, cudaS
   if (D == 3) k_spec_filter<R, 3><<<nb(a.nmodes), 256, 0, st>>>(a);
   else k_spec_filter<R, 2><<<nb(a.nmodes), 256, 0, st>>>(a);
 }
+template <typename R> void launch_gauss_table(void* w, int n, double kfac, double delta, cudaStream_t st) {
+  k_gauss_table<R><<<nb(n), 256, 0, st>>>(static_cast<R*>(w), n, kfac, delta);
+}
 template <typename R> void launch_closure_pt(const LesPhysArgs& a, int D, cudaStream_t st) {
   if (D == 3) k_closure_pt<R, 3><<<nb(a.npts), 256, 0, st>>>(a);
   else k_closure_pt<R, 2><<<nb(a.npts), 256, 0, st>>>(a);
@@ -305,6 +277,7 @@ template <typename R> void launch_dynsmag_mlmm(const LesPhysArgs& a, int D, doub
   template void launch_grad<R>(const LesSpecArgs&, int, cudaStream_t);              \
   template void launch_strain<R>(const LesSpecArgs&, int, cudaStream_t);            \
   template void launch_spec_filter<R>(const LesSpecArgs&, int, cudaStream_t);       \
+  template void launch_gauss_table<R>(void*, int, double, double, cudaStream_t);    \
   template void launch_closure_pt<R>(const LesPhysArgs&, int, cudaStream_t);        \
   template void launch_smag_tensor<R>(const LesPhysArgs&, int, cudaStream_t);       \
   template void launch_sub_products<R>(const LesPhysArgs&, int, cudaStream_t);      \

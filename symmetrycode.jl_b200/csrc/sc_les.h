@@ -35,6 +35,8 @@ struct LesPhysArgs {
 template <typename R> void launch_grad(const LesSpecArgs& a, int D, cudaStream_t st);
 template <typename R> void launch_strain(const LesSpecArgs& a, int D, cudaStream_t st);
 template <typename R> void launch_spec_filter(const LesSpecArgs& a, int D, cudaStream_t st);
+// w[q] = Gaussian of width delta at |k|^2 = q (2 pi / l)^2, q < n (spec_filter's factor)
+template <typename R> void launch_gauss_table(void* w, int n, double kfac, double delta, cudaStream_t st);
 template <typename R> void launch_closure_pt(const LesPhysArgs& a, int D, cudaStream_t st);
 template <typename R> void launch_smag_tensor(const LesPhysArgs& a, int D, cudaStream_t st);
 template <typename R> void launch_sub_products(const LesPhysArgs& a, int D, cudaStream_t st);

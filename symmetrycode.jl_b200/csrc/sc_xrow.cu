@@ -50,6 +50,15 @@ template <typename R> bool xrow_r2c(int N, const XPlainArgs& a, const void* tw, 
     default: return false;
   }
 }
+template <typename R> bool xrow_point(int N, const XPointArgs& a, const void* tw, cudaStream_t st) {
+  if ((a.nin != 6 && a.nin != 9) || (a.nrows & 1)) return false;
+  switch (N) {
+#define SC_CASE(NN, ...) case NN: XRow<R, NN>::point(a, xtab<R>(N, tw), st); return true;
+    SC_SWEEP_SIZES(SC_CASE)
+#undef SC_CASE
+    default: return false;
+  }
+}
 template <typename R>
 bool xrow_vmax(int N, const XPlainArgs& a, const void* tw, unsigned long long* out, cudaStream_t st) {
   if (a.K1 != N / 3 + 1 || (a.nrows & 1)) return false;
@@ -66,6 +75,7 @@ bool xrow_vmax(int N, const XPlainArgs& a, const void* tw, unsigned long long* o
   template bool xrow_ns<R>(int, const XArgs&, const void*, cudaStream_t);                               \
   template bool xrow_c2r<R>(int, const XPlainArgs&, const void*, cudaStream_t);                         \
   template bool xrow_r2c<R>(int, const XPlainArgs&, const void*, cudaStream_t);                         \
+  template bool xrow_point<R>(int, const XPointArgs&, const void*, cudaStream_t);                       \
   template bool xrow_vmax<R>(int, const XPlainArgs&, const void*, unsigned long long*, cudaStream_t);
 SC_INST(float)
 SC_INST(double)

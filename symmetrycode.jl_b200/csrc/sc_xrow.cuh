@@ -25,6 +25,7 @@
 #pragma once
 #include "sc_fft.cuh"
 #include "sc_internal.h"
+#include "sc_closure_pt.cuh"
 #include "sc_xrow.h"
 
 namespace sc {
@@ -449,6 +450,103 @@ k_xr_r2c(const __grid_constant__ XPlainArgs a, const typename V2<R>::T* __restri
 }
 
 // ---------------------------------------------------------------------------
+// closure sweep: c2r of NI fields, the closure's point function, r2c of the six
+// stress components.  Pencil p of a row pair is field p's rows (r, r + 1), so a
+// slot's place holds both rows' value of one point; the six stresses take the
+// places of the first six fields.  Against c2r, point kernel and r2c it spares
+// the write and the read of NI + 6 physical fields (128^3 FP32, six in six out:
+// 66 us in three kernels).
+// ---------------------------------------------------------------------------
+template <typename R, int N, int NI>
+__global__ void __launch_bounds__(32 * XRowCfg<R, N>::wpc(NI), XRowCfg<R, N>::minb(NI, XRowCfg<R, N>::regs_plain))
+k_xr_point(const __grid_constant__ XPointArgs a, const typename V2<R>::T* __restrict__ t1,
+           const typename V2<R>::T* __restrict__ t2) {
+  using C = typename V2<R>::T;
+  using Cfg = XRowCfg<R, N>;
+  constexpr int N1 = Cfg::N1, N2 = Cfg::N2, W = Cfg::W, PS = Cfg::PS, KC = Cfg::KC, K1 = KC + 1, WPC = Cfg::wpc(NI);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31;
+  C* sm = reinterpret_cast<C*>(smem_raw + (threadIdx.x >> 5) * Cfg::slots(NI));
+  const int npair = int(a.nrows >> 1);
+  const int rp0 = (int(blockIdx.x) * WPC + (threadIdx.x >> 5)) * W;
+  if (rp0 >= npair) return;
+#pragma unroll 1
+  for (int it = lane; it < W * NI * N2; it += 32) {
+    const int q = it / N2, j = it - q * N2, p = q / W, w = q - p * W;  // slot q: field p of row pair w
+    const C* ra = static_cast<const C*>(a.in[p]) + 2 * (rp0 + w) * K1;
+    xr_i1<R, N, KC>(ra, ra + K1, rp0 + w < npair, j, t1, sm + q * PS);
+  }
+  __syncwarp();
+  const int w = lane / N1, i = lane - w * N1;
+  const bool act = w < W;
+  C* own = sm + w * PS + i * Cfg::SP;  // this lane's points of field p at own[p W PS + s]
+  if (act) {
+#pragma unroll 1
+    for (int p = 0; p < NI; ++p) {
+      C v[N2];
+      xr_i2<R, N>(sm + (p * W + w) * PS, i, v);
+#pragma unroll
+      for (int s = 0; s < N2; ++s) own[p * W * PS + s] = v[s];
+    }
+    const R d2 = R(a.delta * a.delta), p0 = R(a.p0);
+#pragma unroll 1
+    for (int s = 0; s < N2; ++s) {
+      C z[NI];
+#pragma unroll
+      for (int p = 0; p < NI; ++p) z[p] = own[p * W * PS + s];
+      if constexpr (NI == 6) {
+        R x[6], y[6];
+#pragma unroll
+        for (int p = 0; p < 6; ++p) { x[p] = z[p].x; y[p] = z[p].y; }
+        const R nx = smag_viscosity<R, 3>(d2, x), ny = smag_viscosity<R, 3>(d2, y);
+#pragma unroll
+        for (int p = 0; p < 6; ++p) own[p * W * PS + s] = mk<C>(-R(2) * nx * x[p], -R(2) * ny * y[p]);
+      } else {
+        R G[2][3][3], t[2][3][3];
+#pragma unroll
+        for (int p = 0; p < 9; ++p) { G[0][p % 3][p / 3] = z[p].x; G[1][p % 3][p / 3] = z[p].y; }
+        closure_point<R, 3>(a.kind, d2, p0, G[0], t[0]);
+        closure_point<R, 3>(a.kind, d2, p0, G[1], t[1]);
+        constexpr int PI[6] = {0, 1, 2, 0, 1, 2}, PJ[6] = {0, 1, 2, 1, 2, 0};
+#pragma unroll
+        for (int p = 0; p < 6; ++p) own[p * W * PS + s] = mk<C>(t[0][PI[p]][PJ[p]], t[1][PI[p]][PJ[p]]);
+      }
+    }
+  }
+#pragma unroll 1
+  for (int p = 0; p < 6; ++p) {
+    C v[N2];
+    if (act) {
+#pragma unroll
+      for (int s = 0; s < N2; ++s) v[s] = own[p * W * PS + s];
+    }
+    __syncwarp();
+    if (act) xr_f1<R, N>(v, i, t2, sm + (p * W + w) * PS);
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int it = lane; it < W * 6 * N2; it += 32) {
+    const int q = it / N2, kp = it - q * N2;
+    xr_f2<R, N, KC>(sm + q * PS, kp);
+  }
+  __syncwarp();
+  const R hsc = R(0.5) * R(a.scale);
+  for (int it = lane; it < W * K1; it += 32) {
+    const int ww = it / K1, kx = it - ww * K1;
+    if (rp0 + ww >= npair) break;
+    const int o = 2 * (rp0 + ww) * K1 + kx;
+    const int at = xr_at<R, N>(kx), an = xr_at<R, N>(kx == 0 ? 0 : N - kx);
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+      const C* z = sm + (p * W + ww) * PS;
+      const C x = z[at], y = z[an];
+      static_cast<C*>(a.out[p])[o] = mk<C>(hsc * (x.x + y.x), hsc * (x.y - y.y));
+      static_cast<C*>(a.out[p])[o + K1] = mk<C>(hsc * (x.y + y.y), hsc * (y.x - x.x));
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // max over the physical points of |u|^2 (FP64) of D fields of rows
 // (propose_timestep, src/solver.jl:931-947); *out is the bit pattern of the
 // largest value so far (non-negative doubles order like their bits)
@@ -528,6 +626,8 @@ template <typename R, int N> void XRow<R, N>::init() {
   xr_smem(k_xr_c2r<R, N, N / 2>, s3);
   xr_smem(k_xr_r2c<R, N, N / 3>, s3);
   xr_smem(k_xr_r2c<R, N, N / 2>, s3);
+  xr_smem(k_xr_point<R, N, 6>, Cfg::wpc(6) * Cfg::slots(6));
+  xr_smem(k_xr_point<R, N, 9>, Cfg::wpc(9) * Cfg::slots(9));
   xr_smem(k_xr_vmax<R, N, 2>, s3);
   xr_smem(k_xr_vmax<R, N, 3>, s3);
 }
@@ -574,6 +674,19 @@ template <typename R, int N> void XRow<R, N>::r2c(const XPlainArgs& a, const voi
   const unsigned nb = xr_grid(a.nrows / 2 * a.ncomp, 3 * Cfg::W, wpc);
   if (a.K1 == N / 2 + 1) k_xr_r2c<R, N, N / 2><<<nb, 32 * wpc, wpc * Cfg::slots(3), st>>>(a, t2);
   else k_xr_r2c<R, N, N / 3><<<nb, 32 * wpc, wpc * Cfg::slots(3), st>>>(a, t2);
+}
+
+template <typename R, int N> void XRow<R, N>::point(const XPointArgs& a, const void* tx, cudaStream_t st) {
+  using C = typename V2<R>::T;
+  using Cfg = XRowCfg<R, N>;
+  const C* t1 = static_cast<const C*>(tx);
+  if (a.nin == 6) {
+    constexpr int wpc = Cfg::wpc(6);
+    k_xr_point<R, N, 6><<<xr_grid(a.nrows / 2, Cfg::W, wpc), 32 * wpc, wpc * Cfg::slots(6), st>>>(a, t1, t1 + N);
+  } else {
+    constexpr int wpc = Cfg::wpc(9);
+    k_xr_point<R, N, 9><<<xr_grid(a.nrows / 2, Cfg::W, wpc), 32 * wpc, wpc * Cfg::slots(9), st>>>(a, t1, t1 + N);
+  }
 }
 
 template <typename R, int N>

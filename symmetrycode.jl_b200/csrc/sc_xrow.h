@@ -11,6 +11,7 @@ template <typename R, int N> struct XRow {
   static void ns(const XArgs& a, const void* tx, cudaStream_t st);
   static void c2r(const XPlainArgs& a, const void* tx, cudaStream_t st);
   static void r2c(const XPlainArgs& a, const void* tx, cudaStream_t st);
+  static void point(const XPointArgs& a, const void* tx, cudaStream_t st);
   static void vmax(const XPlainArgs& a, const void* tx, unsigned long long* out, cudaStream_t st);
 };
 
@@ -19,6 +20,7 @@ template <typename R> bool xrow_init(int N);
 template <typename R> bool xrow_ns(int N, const XArgs& a, const void* tw, cudaStream_t st);
 template <typename R> bool xrow_c2r(int N, const XPlainArgs& a, const void* tw, cudaStream_t st);
 template <typename R> bool xrow_r2c(int N, const XPlainArgs& a, const void* tw, cudaStream_t st);
+template <typename R> bool xrow_point(int N, const XPointArgs& a, const void* tw, cudaStream_t st);
 template <typename R>
 bool xrow_vmax(int N, const XPlainArgs& a, const void* tw, unsigned long long* out, cudaStream_t st);
 
