@@ -3,24 +3,27 @@
 // X(N, xf1, xf2, xd1, xd2, c1, c2): N = xf1 * xf2 splits the x rows in FP32
 // (xf1 lanes of a warp hold xf2 points each between the inverse and the
 // forward transform), N = xd1 * xd2 in FP64, N = c1 * c2 the column sweeps
-// (radix c1 first).  Chosen so that xf1 fills the 32 lanes (a warp takes
-// 32 / xf1 row pairs) and 3 * (32 / xf1) * xf2, the work items of the other
-// radix pass, fills whole rounds of 32; the points per lane are what the
-// registers hold (about 6 values per point), so FP64 takes fewer of them.
+// (radix c1 first).  Few points a lane keep the slots small (32 / xf1 row pairs
+// a warp, 4 to 9 slots each) and more warps resident, which is worth more than
+// full rounds of work items: 128 FP32, product sweep of 2 GB 743 us as 8 x 16 and
+// 578 as 16 x 8, Clark's closure sweep 54 and 38 us; 256 FP64 625 us as 16 x 16
+// and 570 as 32 x 8; 120 FP32 801 us as 8 x 15 and 632 as 15 x 8.  Below that the
+// sweeps of a grid are short and the wider split starts faster (64 FP32, 64^3:
+// 5.8 us as 8 x 8, 5.1 as 16 x 4).
 // Sizes below 32 keep the shared-memory engine of sc_kernels.cu.
 #pragma once
 
 #define SC_SWEEP_SIZES_A(X) \
-  X(32, 8, 4, 8, 4, 8, 4) X(36, 6, 6, 6, 6, 6, 6) X(40, 8, 5, 8, 5, 8, 5) X(48, 6, 8, 6, 8, 8, 6) \
-  X(60, 6, 10, 6, 10, 10, 6) X(64, 8, 8, 8, 8, 8, 8) X(72, 8, 9, 8, 9, 9, 8) X(80, 8, 10, 8, 10, 10, 8) \
-  X(90, 10, 9, 10, 9, 10, 9) X(96, 8, 12, 8, 12, 12, 8)
+  X(32, 16, 2, 16, 2, 8, 4) X(36, 12, 3, 12, 3, 6, 6) X(40, 20, 2, 20, 2, 8, 5) X(48, 12, 4, 12, 4, 8, 6) \
+  X(60, 15, 4, 15, 4, 10, 6) X(64, 16, 4, 16, 4, 8, 8) X(72, 18, 4, 18, 4, 9, 8) X(80, 16, 5, 16, 5, 10, 8) \
+  X(90, 15, 6, 15, 6, 10, 9) X(96, 16, 6, 16, 6, 12, 8)
 #define SC_SWEEP_SIZES_B(X) \
-  X(120, 8, 15, 15, 8, 12, 10) X(128, 8, 16, 16, 8, 16, 8) X(160, 16, 10, 16, 10, 16, 10) \
-  X(180, 15, 12, 15, 12, 15, 12) X(192, 16, 12, 16, 12, 16, 12) X(240, 16, 15, 16, 15, 16, 15) \
-  X(256, 16, 16, 16, 16, 16, 16)
+  X(120, 15, 8, 15, 8, 12, 10) X(128, 16, 8, 16, 8, 16, 8) X(160, 20, 8, 20, 8, 16, 10) \
+  X(180, 20, 9, 20, 9, 15, 12) X(192, 24, 8, 24, 8, 16, 12) X(240, 30, 8, 30, 8, 16, 15) \
+  X(256, 32, 8, 32, 8, 16, 16)
 #define SC_SWEEP_SIZES_C(X) \
-  X(270, 30, 9, 30, 9, 18, 15) X(320, 32, 10, 32, 10, 20, 16) X(360, 15, 24, 30, 12, 20, 18) \
-  X(384, 32, 12, 32, 12, 24, 16) X(512, 32, 16, 32, 16, 32, 16)
+  X(270, 30, 9, 27, 10, 18, 15) X(320, 32, 10, 32, 10, 20, 16) X(360, 24, 15, 24, 15, 20, 18) \
+  X(384, 24, 16, 24, 16, 24, 16) X(512, 32, 16, 32, 16, 32, 16)
 #define SC_SWEEP_SIZES_D(X) \
   X(540, 30, 18, 30, 18, 27, 20) X(640, 32, 20, 32, 20, 32, 20) X(720, 30, 24, 30, 24, 30, 24) \
   X(768, 32, 24, 32, 24, 32, 24) X(810, 30, 27, 30, 27, 27, 30) X(1024, 32, 32, 32, 32, 32, 32)
