@@ -187,6 +187,24 @@ int plan_alloc(sc_plan* p, void** out, size_t bytes) {
   return SC_OK;
 }
 
+// The plan's small buffers in one allocation (each costs a fraction of a
+// millisecond): twiddles, those of a smaller size (the pair table of 810
+// included), scalars, shell sums, the error word.
+int plan_tables(sc_plan* p) {
+  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t tw = up(sc::twiddle_buffer_bytes(p->n, p->esz));
+  const size_t twr = p->D == 3 ? up(3 * (size_t)p->n * p->esz + sc::xpair810_twiddle_bytes()) : 0;
+  const size_t shells = up((p->kc + 3) * sizeof(double));
+  const int rc = plan_alloc(p, &p->tw, tw + twr + shells + 512);
+  if (rc) return rc;
+  char* b = static_cast<char*>(p->tw) + tw;
+  if (twr) p->twr = b;
+  p->shells = reinterpret_cast<double*>(b + twr);
+  p->dscal = reinterpret_cast<double*>(b + twr + shells);
+  p->err = reinterpret_cast<int*>(b + twr + shells + 256);
+  return SC_OK;
+}
+
 void plan_free(sc_plan* p) {
   if (p->g_rk4) cudaGraphExecDestroy(p->g_rk4);
   if (p->g_wray) cudaGraphExecDestroy(p->g_wray);
@@ -1188,9 +1206,7 @@ int sc_plan_create(sc_plan** out, int D, int n, double l, int dtype, size_t* wor
   int rc = SC_OK;
   bool ok = (dtype == SC_FLOAT64) ? sc::init_kernels<double>(n) : sc::init_kernels<float>(n);
   if (!ok) { rc = fail(SC_ERR_CUDA, "kernel attribute setup failed for n=%d", n); goto bad; }
-  if ((rc = plan_alloc(p, &p->tw, sc::twiddle_buffer_bytes(n, p->esz)))) goto bad;
-  // a smaller size's buffer, the pair table of 810 included
-  if (D == 3 && (rc = plan_alloc(p, &p->twr, 3 * (size_t)n * p->esz + sc::xpair810_twiddle_bytes()))) goto bad;
+  if ((rc = plan_tables(p))) goto bad;
   for (int c = 0; c < D; ++c) {
     if ((rc = plan_alloc(p, &p->U[c], p->csz * p->esz))) goto bad;
     if ((rc = plan_alloc(p, &p->ACC[c], p->csz * p->esz))) goto bad;
@@ -1203,9 +1219,6 @@ int sc_plan_create(sc_plan** out, int D, int n, double l, int dtype, size_t* wor
   }
   for (int c = 0; c < D; ++c)
     if ((rc = plan_alloc(p, &p->cc[c], plane * p->esz))) goto bad;
-  if ((rc = plan_alloc(p, (void**)&p->dscal, 16 * sizeof(double)))) goto bad;
-  if ((rc = plan_alloc(p, (void**)&p->shells, (p->kc + 3) * sizeof(double)))) goto bad;
-  if ((rc = plan_alloc(p, (void**)&p->err, sizeof(int)))) goto bad;
   if (cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking) != cudaSuccess) {
     rc = fail(SC_ERR_CUDA, "stream creation failed");
     goto bad;
@@ -1570,18 +1583,17 @@ int sc_closure_create(sc_closure** out, sc_plan* p, int kind, double delta, cons
     for (int c = 0; c < D && !rc; ++c) rc = A(&cl->ph4[c], pb);
     for (int c = 0; c < 12 && !rc; ++c) rc = A(&cl->cb[c], plane);
     for (int c = 0; c < 12 && !rc && D == 3; ++c) rc = A(&cl->bb[c], mid);
-    if (!rc) rc = A((void**)&cl->dsum, 4 * sizeof(double));
     // Bardina and dynamic Smagorinsky filter at one width only: its Gaussian at
     // every |k|^2 of the cube, read by the inverse z sweeps (y in 2D)
-    if (!rc && (kind == sc::kBardina || kind == sc::kDynSmagorinsky) && sc::sweep_size(p->n, p->dtype == SC_FLOAT32)) {
-      const int nq = D * p->kc * p->kc + 1;
+    const bool table = (kind == sc::kBardina || kind == sc::kDynSmagorinsky) && sc::sweep_size(p->n, p->dtype == SC_FLOAT32);
+    const int nq = table ? D * p->kc * p->kc + 1 : 0;
+    if (!rc) rc = A((void**)&cl->dsum, 256 + nq * (p->esz / 2));  // four scalars, then the table
+    if (!rc && table) {
       const double width = kind == sc::kBardina ? cl->prm[0] * delta : 2.0 * delta, kfac = 2.0 * M_PI / p->l;
-      rc = A(&cl->wtab, nq * (p->esz / 2));
-      if (!rc) {
-        if (p->dtype == SC_FLOAT64) sc::launch_gauss_table<double>(cl->wtab, nq, kfac, width, 0);
-        else sc::launch_gauss_table<float>(cl->wtab, nq, kfac, width, 0);
-        if (cudaStreamSynchronize(0) != cudaSuccess) rc = fail(SC_ERR_CUDA, "test filter table");
-      }
+      cl->wtab = cl->dsum + 256 / sizeof(double);
+      if (p->dtype == SC_FLOAT64) sc::launch_gauss_table<double>(cl->wtab, nq, kfac, width, 0);
+      else sc::launch_gauss_table<float>(cl->wtab, nq, kfac, width, 0);
+      if (cudaStreamSynchronize(0) != cudaSuccess) rc = fail(SC_ERR_CUDA, "test filter table");
     }
   }
   if (rc) {
