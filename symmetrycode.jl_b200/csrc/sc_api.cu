@@ -188,12 +188,12 @@ int plan_alloc(sc_plan* p, void** out, size_t bytes) {
 }
 
 // The plan's small buffers in one allocation (each costs a fraction of a
-// millisecond): twiddles, those of a smaller size (the pair table of 810
-// included), scalars, shell sums, the error word.
+// millisecond): twiddles, those of a smaller size (810's own tables included),
+// scalars, shell sums, the error word.
 int plan_tables(sc_plan* p) {
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t tw = up(sc::twiddle_buffer_bytes(p->n, p->esz));
-  const size_t twr = p->D == 3 ? up(3 * (size_t)p->n * p->esz + sc::xpair810_twiddle_bytes()) : 0;
+  const size_t twr = p->D == 3 ? up(3 * (size_t)p->n * p->esz + sc::xpair810_twiddle_bytes() + sc::X4Tab::SIZE * 8) : 0;
   const size_t shells = up((p->kc + 3) * sizeof(double));
   const int rc = plan_alloc(p, &p->tw, tw + twr + shells + 512);
   if (rc) return rc;
@@ -238,6 +238,18 @@ std::vector<unsigned char> twiddle_image(int n) {
     for (int q = 0; q < n; ++q) {
       t1[q] = h[(q / n2) * (q % n2)];
       t1[n + q] = h[(q / n1) * (q % n1)];
+    }
+  }
+  if (n == 810 && sizeof(R) == 4) {
+    C* t4 = reinterpret_cast<C*>(img.data() + sc::twiddle_x4_offset(n, sizeof(C)));
+    for (int s = 0; s < 10; ++s)
+      for (int q = 0; q < 9; ++q) t4[sc::X4Tab::A + 9 * s + q] = h[9 * q * s % n];
+    for (int s = 0; s < 9; ++s) {
+      for (int t = 0; t < 90; ++t) {
+        t4[sc::X4Tab::B + 90 * s + t] = h[(t % 9) * (t / 9 + 10 * s) % n];
+        t4[sc::X4Tab::F + 90 * s + t] = h[t * s % n];
+      }
+      for (int q = 0; q < 10; ++q) t4[sc::X4Tab::G + 10 * s + q] = h[9 * q * s % n];
     }
   }
   return img;

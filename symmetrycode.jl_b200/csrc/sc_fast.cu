@@ -168,7 +168,7 @@ k_xsweep4(const XArgs a, const float2* __restrict__ tw) {
     const int q = t / 9;
     C w[10];
 #pragma unroll
-    for (int sa = 1; sa < 10; ++sa) { const C v = __ldg(&tw[9 * q * sa]); w[sa] = make_float2(v.x, -v.y); }
+    for (int sa = 1; sa < 10; ++sa) { const C v = __ldg(tw + X4Tab::A + 9 * sa + q); w[sa] = make_float2(v.x, -v.y); }
 #pragma unroll 1
     for (int j = 0; j < 3; ++j) {
       // A: u1, u2 of row r; A': u1, u2 of row r'; B: u3 of rows r and r'
@@ -193,7 +193,7 @@ k_xsweep4(const XArgs a, const float2* __restrict__ tw) {
     const int sa = t / 9, m2 = t - 9 * sa;
     C w[9];
 #pragma unroll
-    for (int sb = 0; sb < 9; ++sb) { const C v = __ldg(&tw[m2 * (sa + 10 * sb)]); w[sb] = make_float2(v.x, -v.y); }
+    for (int sb = 0; sb < 9; ++sb) { const C v = __ldg(tw + X4Tab::B + 90 * sb + t); w[sb] = make_float2(v.x, -v.y); }
 #pragma unroll 1
     for (int j = 0; j < 3; ++j) {
       const C* xs = reg0 + j * PS + 89 * sa + m2;
@@ -214,7 +214,7 @@ k_xsweep4(const XArgs a, const float2* __restrict__ tw) {
   C wf[9];
   if (t < 90) {
 #pragma unroll
-    for (int s = 1; s < 9; ++s) wf[s] = __ldg(&tw[t * s]);
+    for (int s = 1; s < 9; ++s) wf[s] = __ldg(tw + X4Tab::F + 90 * s + t);
     C v[9];
     const C* ya = reg1 + 9 * t;
 #pragma unroll
@@ -245,7 +245,7 @@ k_xsweep4(const XArgs a, const float2* __restrict__ tw) {
     C w2[9];
     if (t < 90) {
 #pragma unroll
-      for (int s = 1; s < 9; ++s) w2[s] = __ldg(&tw[9 * q * s]);
+      for (int s = 1; s < 9; ++s) w2[s] = __ldg(tw + X4Tab::G + 10 * s + q);
     }
 #pragma unroll 1
     for (int g = 0; g < 2; ++g) {
@@ -842,8 +842,9 @@ bool launch_xsweep810(const XArgs& a, const void* tw, cudaStream_t st) {
     return true;
   }
   const unsigned nb4 = unsigned((a.nrows + 1) / 2);
-  if (a.K1in == 271 && a.K1out == 271) k_xsweep4<true><<<nb4, X4Cfg::NT, X4Cfg::SMEM, st>>>(a, t2);
-  else k_xsweep4<false><<<nb4, X4Cfg::NT, X4Cfg::SMEM, st>>>(a, t2);
+  const float2* t4 = reinterpret_cast<const float2*>(static_cast<const char*>(tw) + twiddle_x4_offset(810, 8));
+  if (a.K1in == 271 && a.K1out == 271) k_xsweep4<true><<<nb4, X4Cfg::NT, X4Cfg::SMEM, st>>>(a, t4);
+  else k_xsweep4<false><<<nb4, X4Cfg::NT, X4Cfg::SMEM, st>>>(a, t4);
   return true;
 }
 

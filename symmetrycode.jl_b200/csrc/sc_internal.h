@@ -187,7 +187,20 @@ void launch_xpair810(const XArgs& a, const void* twp_table, int minb, cudaStream
 inline size_t twiddle_x_offset(int n, size_t esz) {
   return (size_t)n * esz + (esz == 8 && n == 810 ? xpair810_twiddle_bytes() : 0);
 }
-inline size_t twiddle_buffer_bytes(int n, size_t esz) { return twiddle_x_offset(n, esz) + 2 * (size_t)n * esz; }
+// Then, for FP32 n = 810, the tables of the three-level x sweep (X4Tab).
+inline size_t twiddle_x4_offset(int n, size_t esz) { return twiddle_x_offset(n, esz) + 2 * (size_t)n * esz; }
+// Twiddles of the 810 x sweep's passes, indexed as its threads t are (from the
+// plain table a warp's load touched up to 27 lines; 102 500 rows 899 -> 857 us):
+struct X4Tab {
+  static constexpr int A = 0;             // [s][q]: 9 q s, s = 1..9, q = 0..8
+  static constexpr int B = A + 90;        // [s][t]: m2 (sa + 10 s), s = 0..8, t = 9 sa + m2
+  static constexpr int F = B + 9 * 90;    // [s][t]: t s, s = 1..8
+  static constexpr int G = F + 9 * 90;    // [s][q]: 9 q s, s = 1..8, q = 0..9
+  static constexpr int SIZE = G + 90;
+};
+inline size_t twiddle_buffer_bytes(int n, size_t esz) {
+  return twiddle_x4_offset(n, esz) + (esz == 8 && n == 810 ? X4Tab::SIZE * esz : 0);
+}
 template <typename R> bool init_kernels(int N);
 template <typename R> void launch_twothirds_full(const PackArgs& a, cudaStream_t st);  // in place on a.dst
 template <typename R> void launch_project_full(const PackArgs& a, double kfac, cudaStream_t st);
