@@ -129,21 +129,34 @@ struct ConvOut {
 // The epilogue may lag the MMAs by up to four steps (the accumulator ring and
 // the four step barriers), so its latency overlaps the tensor pipe's work.  A
 // change of z-plane ends the run with a CTA barrier and restages.
-constexpr int kSlots = 5;
+//
+// FUSED: one launch does a whole split-precision layer.  The high and low parts
+// of the input rows and of the weights are staged side by side, and each (dz, dx,
+// 16 channels) issues three MMAs: A_hi W_hi into the accumulators above,
+// A_lo W_hi and A_hi W_lo into a second set of eight blocks (the small terms
+// round at their own size), added at read-out.  Against three launches the rows
+// are staged once instead of three times and the FP32 sums never leave the chip
+// (64^3, 32 -> 32, FP16: 155 us in three passes).  With the doubled rows and
+// weights there is room for a ring of four rows, and only where the rows are 64
+// long or 16 channels wide (conv_fused_fits).
 constexpr int kConvThreads = 384;
+template <bool FUSED> constexpr int conv_slots() { return FUSED ? 4 : 5; }
 
-template <int KN, int CP, int COP, int MODE, bool F16>
+template <int KN, int CP, int COP, int MODE, bool F16, bool FUSED = false>
 __global__ void __launch_bounds__(kConvThreads, 1)
-k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__ wgt,
+k_conv3(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvMaps maps_lo,
+        const __nv_bfloat16* __restrict__ wgt, const __nv_bfloat16* __restrict__ wgt_lo,
         const float* __restrict__ bias, const ConvOut out, int* __restrict__ err, long long wait_limit) {
   constexpr int kRowPlane = row_plane<KN>();
+  constexpr int kSlots = conv_slots<FUSED>();
+  constexpr int NP = FUSED ? 2 : 1;        // operand parts staged
   constexpr int CPC = CP / 8;              // 16-byte channel chunks
-  constexpr int PLANE_ROW = CPC * kRowPlane;
+  constexpr int PLANE_ROW = NP * CPC * kRowPlane;
   constexpr int SIN = 3 * kSlots * PLANE_ROW;  // [zr][slot] staged rows
   constexpr int NS = 3 * COP;              // stacked rows per k-chunk plane: the three dy taps
-  constexpr int SW = 9 * CPC * NS * 16;
+  constexpr int SW1 = 9 * CPC * NS * 16, SW = NP * SW1;
   constexpr uint32_t IDESC = make_idesc<3 * COP, F16>();
-  constexpr uint32_t kTmemCols = 8 * COP;  // eight accumulator blocks
+  constexpr uint32_t kTmemCols = NP * 8 * COP;  // eight accumulator blocks (each part's terms)
   extern __shared__ __align__(128) unsigned char sm[];
   unsigned char* s_in = sm;
   unsigned char* s_w = sm + SIN;
@@ -164,11 +177,12 @@ k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__
   // stacked weights: chunk ((dz 3 + dx) CPC + kc) NS + j COP + co holds tap
   // (dz, dy index 2 - j, dx) of the [27][CPC][COP] layout (dy index 0, 1, 2
   // for dy = -1, 0, +1), j = 0, 1, 2 for the output rows y' - 1, y', y' + 1
-  for (int d = tid; d < SW / 16; d += blockDim.x) {
+  for (int d = tid; d < SW1 / 16; d += blockDim.x) {
     const int co = d % COP, j = (d % NS) / COP, kc = (d / NS) % CPC, g = d / (NS * CPC);
     const int dyi = 2 - j;
     const int src = (((g / 3) * 9 + dyi * 3 + g % 3) * CPC + kc) * COP + co;
     reinterpret_cast<uint4*>(s_w)[d] = __ldg(reinterpret_cast<const uint4*>(wgt) + src);
+    if (FUSED) reinterpret_cast<uint4*>(s_w + SW1)[d] = __ldg(reinterpret_cast<const uint4*>(wgt_lo) + src);
   }
   constexpr bool kBias = MODE == kGelu || MODE == kGeluSave || MODE == kTau || MODE == kGeluSplit || MODE == kTauSplit;
   constexpr bool kTauOut = MODE == kTau || MODE == kTauSplit;
@@ -237,6 +251,22 @@ k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__
 #pragma unroll
       for (int c = 0; c < 16; ++c) v[c] += w[c];
     }
+    if (FUSED) {  // the small terms' blocks
+      float w[16];
+      const uint32_t tb = ta + uint32_t(8 * COP);
+      tmem_ld<16>(tb, w);
+      tmem_zero16(tb);
+      if (blk < 2) {
+        float x[16];
+        const uint32_t tc = tb + uint32_t(6 * COP);
+        tmem_ld<16>(tc, x);
+        tmem_zero16(tc);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) w[c] += x[c];
+      }
+#pragma unroll
+      for (int c = 0; c < 16; ++c) v[c] += w[c];
+    }
   };
   // bias + activation + store of row prow (z KN + y) from the read-out values
   auto epilogue = [&](int prow, const float* v) {
@@ -262,9 +292,12 @@ k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__
 #pragma unroll
       for (int c = 0; c < 6; ++c) out.tau.p[c][vox] = v[c] + bia[c];
     } else if (MODE == kTauSplit) {
-      const float4* pl = reinterpret_cast<const float4*>(out.pre + vox * COP);
-      const float4 p0 = pl[0], p1 = pl[1];
-      const float pv[6] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y};
+      float pv[6] = {};
+      if (!FUSED) {
+        const float4* pl = reinterpret_cast<const float4*>(out.pre + vox * COP);
+        const float4 p0 = pl[0], p1 = pl[1];
+        pv[0] = p0.x; pv[1] = p0.y; pv[2] = p0.z; pv[3] = p0.w; pv[4] = p1.x; pv[5] = p1.y;
+      }
 #pragma unroll
       for (int c = 0; c < 6; ++c) out.tau.p[c][vox] = (v[c] + pv[c]) * out.scale + bia[c];
     } else if (MODE == kGeluSplit) {
@@ -273,7 +306,7 @@ k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__
       __align__(16) __half lo[16];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float4 p = pl[j];
+        const float4 p = FUSED ? make_float4(0.f, 0.f, 0.f, 0.f) : pl[j];
         const float h[4] = {(v[4 * j] + p.x) * out.scale + bia[4 * j], (v[4 * j + 1] + p.y) * out.scale + bia[4 * j + 1],
                             (v[4 * j + 2] + p.z) * out.scale + bia[4 * j + 2],
                             (v[4 * j + 3] + p.w) * out.scale + bia[4 * j + 3]};
@@ -315,19 +348,20 @@ k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__
   auto slot_of = [](int yv) { return (yv + KN) % kSlots; };
   auto tma_row = [&](int z, int yv) {
     const int sl = slot_of(yv), yy = (yv + KN) % KN;
-    // bytes delivered: 3 rows x CP/8 boxes of (KN + 2) 16-byte voxels (the
+    // bytes delivered: (NP parts of) 3 rows x CP/8 boxes of (KN + 2) 16-byte voxels (the
     // planes' padding to 128 bytes is not written)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(staged + sl)),
-                 "r"(3 * CPC * (KN + 2) * 16)
+                 "r"(NP * 3 * CPC * (KN + 2) * 16)
                  : "memory");
     for (int zr = 0; zr < 3; ++zr) {
       const int zz = (z + zr - 1 + KN) % KN;
-      for (int c = 0; c < CPC; ++c) {
+      for (int c = 0; c < NP * CPC; ++c) {
+        const uint64_t map = reinterpret_cast<uint64_t>(c < CPC ? &maps.m[c] : &maps_lo.m[c - CPC]);
         unsigned char* dst = s_in + (zr * kSlots + sl) * PLANE_ROW + c * kRowPlane;
         asm volatile(
             "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
             "[%6];" ::"r"(smem_u32(dst)),
-            "l"(reinterpret_cast<uint64_t>(&maps.m[c])), "r"(0), "r"(-1), "r"(yy), "r"(zz), "r"(smem_u32(staged + sl))
+            "l"(map), "r"(0), "r"(-1), "r"(yy), "r"(zz), "r"(smem_u32(staged + sl))
             : "memory");
       }
     }
@@ -337,11 +371,14 @@ k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__
   auto patch_row = [&](int yv) -> bool {
     const int sl = slot_of(yv);
     const bool w = __all_sync(0xffffffffu, wait(staged + sl, (spar >> sl) & 1u));
-    if (w && lane < 3 * CPC * 2) {
-      const int zr = lane / (2 * CPC), c = (lane / 2) % CPC, side = lane & 1;
-      unsigned char* plane = s_in + (zr * kSlots + sl) * PLANE_ROW + c * kRowPlane;
-      const uint4 v = reinterpret_cast<const uint4*>(plane)[side ? 1 : KN];
-      reinterpret_cast<uint4*>(plane)[side ? KN + 1 : 0] = v;
+    if (w) {
+#pragma unroll
+      for (int e = lane; e < 3 * NP * CPC * 2; e += 32) {
+        const int zr = e / (2 * NP * CPC), c = (e / 2) % (NP * CPC), side = e & 1;
+        unsigned char* plane = s_in + (zr * kSlots + sl) * PLANE_ROW + c * kRowPlane;
+        const uint4 v = reinterpret_cast<const uint4*>(plane)[side ? 1 : KN];
+        reinterpret_cast<uint4*>(plane)[side ? KN + 1 : 0] = v;
+      }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     return w;
@@ -366,7 +403,7 @@ k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__
     if (tid == 32)
       for (int yv = y0 - 1; yv <= min(y0 + 2, y1 + 1); ++yv) tma_row(z, yv);
     if (is_epi)
-      for (int q = 0; q < 8; ++q) tmem_zero16(tmem + (uint32_t(lane_base) << 16) + uint32_t(q * COP + ecol0));
+      for (int q = 0; q < 8 * NP; ++q) tmem_zero16(tmem + (uint32_t(lane_base) << 16) + uint32_t(q * COP + ecol0));
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
@@ -396,6 +433,10 @@ k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__
           const uint64_t da = DA0 + sa + uint32_t(dz * kSlots * (PLANE_ROW >> 4) + dx + 2 * h * (kRowPlane >> 4));
           const uint64_t db = DB0 + uint32_t(((dz * 3 + dx) * CPC + 2 * h) * NS);
           mma_bf16_acc(dcol, da, db, IDESC);
+          if (FUSED) {
+            mma_bf16_acc(dcol + uint32_t(8 * COP), da + uint32_t(CPC * (kRowPlane >> 4)), db, IDESC);
+            mma_bf16_acc(dcol + uint32_t(8 * COP), da, db + uint32_t(SW1 >> 4), IDESC);
+          }
         }
         mma_commit(cbar + (kk & 3));
         last_k = kk;
@@ -428,11 +469,11 @@ k_conv3(const __grid_constant__ ConvMaps maps, const __nv_bfloat16* __restrict__
             if (lane == 0) tin &= ~(1u << slot_of(yv + 1));
           }
         }
-        // copy input row yv + 4 into the slot input row yv - 1 left, once step
-        // yv - 1 (its last reader) is done
-        if (mine && yv + 4 <= y1 + 1) {
+        // copy input row yv + kSlots - 1 into the slot input row yv - 1 left, once
+        // step yv - 1 (its last reader) is done (the first four rows are under way)
+        if (mine && yv + kSlots - 1 <= y1 + 1 && (kSlots == 5 || i > 0)) {
           if (i > 0) mine = __all_sync(0xffffffffu, wait(cbar + ((kk - 1) & 3), uint32_t((kk - 1) >> 2) & 1u));
-          if (mine && lane == 0) tma_row(z, yv + 4);
+          if (mine && lane == 0) tma_row(z, yv + kSlots - 1);
         }
       }
       if (!mine) fail();
@@ -583,49 +624,72 @@ __global__ void k_gin_planar(const float* __restrict__ gin, const GinPtrs o, lon
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-template <int KN, int CP, int COP> static size_t conv_smem() {
-  // + the mbarriers (4 steps, 2 x kSlots rows, 6 blocks), the TMEM slot and the abort flag
-  return size_t(3 * kSlots) * (CP / 8) * row_plane<KN>() + size_t(27) * (CP / 8) * COP * 16 + 192;
+template <int KN, int CP, int COP, bool FUSED = false> constexpr size_t conv_smem() {
+  // + the mbarriers (4 steps, 2 x slots rows, 6 blocks), the TMEM slot and the abort flag
+  return (FUSED ? 2 : 1) * (size_t(3 * conv_slots<FUSED>()) * (CP / 8) * row_plane<KN>() + size_t(27) * (CP / 8) * COP * 16) +
+         192;
 }
+template <int KN, int CP, int COP> constexpr bool conv_fused_fits() { return conv_smem<KN, CP, COP, true>() <= 232448; }
 
-template <int KN, int CP, int COP, int MODE, bool F16 = false> static void conv_attr() {
-  cudaFuncSetAttribute(k_conv3<KN, CP, COP, MODE, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       int(conv_smem<KN, CP, COP>()));
+template <int KN, int CP, int COP, int MODE, bool F16 = false, bool FUSED = false> static void conv_attr() {
+  cudaFuncSetAttribute(k_conv3<KN, CP, COP, MODE, F16, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       int(conv_smem<KN, CP, COP, FUSED>()));
+}
+// the launches of a split-precision layer: one, or three passes
+template <int KN, int CP, int COP, int FIN, bool F16> static void conv_split_attr() {
+  constexpr int last = FIN == kAccum ? kLinear : FIN;  // nothing to add to in one launch
+  if constexpr (conv_fused_fits<KN, CP, COP>()) {
+    conv_attr<KN, CP, COP, last, F16, true>();
+  } else {
+    conv_attr<KN, CP, COP, kLinear, F16>();
+    conv_attr<KN, CP, COP, kAccum, F16>();
+    conv_attr<KN, CP, COP, FIN, F16>();
+  }
 }
 
 // in: channels-last 16-bit input (BF16, or FP16 when F16); w: packed 16-bit
 // weights of the same type.  The tensor maps are encoded with the BF16 element
 // type for both: a bulk tensor copy moves 16-bit elements without converting
 // them, and its zero fill is the all-zero bit pattern, +0 in either type.
-template <int KN, int CP, int COP, int MODE, bool F16 = false>
+// FUSED: in_lo and w_lo are the low parts.
+template <int KN, int CP, int COP, int MODE, bool F16 = false, bool FUSED = false>
 static void conv_launch(int grid, const void* in, const void* w, const float* b, const ConvOut& o, int* err,
-                        long long wait_limit, cudaStream_t st) {
+                        long long wait_limit, cudaStream_t st, const void* in_lo = nullptr, const void* w_lo = nullptr) {
   // one map per 8-channel chunk of the channels-last input [z][y][x][CP]:
   // dims (8 channels, x, y, z), boxes of 8 channels x (KN + 2) voxels of one row
-  ConvMaps maps{};
+  ConvMaps maps{}, lo{};
   const unsigned long long dims[4] = {8, KN, KN, KN};
   const unsigned long long str[3] = {CP * 2ull, KN * CP * 2ull, (unsigned long long)KN * KN * CP * 2ull};
   const unsigned box[4] = {8, KN + 2, 1, 1};
   bool enc = true;
-  for (int c = 0; c < CP / 8; ++c)
+  for (int c = 0; c < CP / 8; ++c) {
     enc = enc && tma_encode_bf16_4d(&maps.m[c], static_cast<const unsigned char*>(in) + 16 * c, dims, str, box);
+    if (FUSED)
+      enc = enc && tma_encode_bf16_4d(&lo.m[c], static_cast<const unsigned char*>(in_lo) + 16 * c, dims, str, box);
+  }
   if (!enc) {  // no tensor-map encoder: report it through the closure's error flag
     k_set_flag<<<1, 1, 0, st>>>(err);
     return;
   }
-  k_conv3<KN, CP, COP, MODE, F16><<<grid, kConvThreads, conv_smem<KN, CP, COP>(), st>>>(
-      maps, static_cast<const __nv_bfloat16*>(w), b, o, err, wait_limit);
+  k_conv3<KN, CP, COP, MODE, F16, FUSED><<<grid, kConvThreads, conv_smem<KN, CP, COP, FUSED>(), st>>>(
+      maps, lo, static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(w_lo), b, o, err, wait_limit);
 }
 
-// One layer in split precision: three passes A_hi W_hi (kLinear), A_lo W_hi
-// (kAccum) and A_hi W_lo (FIN), all accumulating in the FP32 buffer o.pre.  The
-// dropped A_lo W_lo term is below the representation error of the parts.
+// One layer in split precision: one fused launch where its operands fit, else
+// three passes A_hi W_hi (kLinear), A_lo W_hi (kAccum) and A_hi W_lo (FIN), all
+// accumulating in the FP32 buffer o.pre.  The dropped A_lo W_lo term is below the
+// representation error of the parts.
 template <int KN, int CP, int COP, int FIN, bool F16>
 static void conv_split(int grid, const void* in_h, const void* in_l, const void* w_h, const void* w_l, const float* b,
                        const ConvOut& o, int* err, long long wait_limit, cudaStream_t st) {
-  conv_launch<KN, CP, COP, kLinear, F16>(grid, in_h, w_h, nullptr, o, err, wait_limit, st);
-  conv_launch<KN, CP, COP, kAccum, F16>(grid, in_l, w_h, nullptr, o, err, wait_limit, st);
-  conv_launch<KN, CP, COP, FIN, F16>(grid, in_h, w_l, b, o, err, wait_limit, st);
+  if constexpr (conv_fused_fits<KN, CP, COP>()) {
+    conv_launch<KN, CP, COP, FIN == kAccum ? kLinear : FIN, F16, true>(grid, in_h, w_h, b, o, err, wait_limit, st, in_l,
+                                                                       w_l);
+  } else {
+    conv_launch<KN, CP, COP, kLinear, F16>(grid, in_h, w_h, nullptr, o, err, wait_limit, st);
+    conv_launch<KN, CP, COP, kAccum, F16>(grid, in_l, w_h, nullptr, o, err, wait_limit, st);
+    conv_launch<KN, CP, COP, FIN, F16>(grid, in_h, w_l, b, o, err, wait_limit, st);
+  }
 }
 
 bool cnn_supported(int n, int D) { return (n == 64 || n == 128) && D == 3; }
@@ -644,18 +708,12 @@ template <int KN> static void cnn_init_n() {
   conv_attr<KN, 32, 32, kLinear>();
   conv_attr<KN, 32, 16, kLinear>();
   // split precision: FP16 forward passes, BF16 input-gradient passes
-  conv_attr<KN, 16, 32, kLinear, true>();
-  conv_attr<KN, 16, 32, kAccum, true>();
-  conv_attr<KN, 16, 32, kGeluSplit, true>();
-  conv_attr<KN, 32, 32, kLinear, true>();
-  conv_attr<KN, 32, 32, kAccum, true>();
-  conv_attr<KN, 32, 32, kGeluSplit, true>();
-  conv_attr<KN, 32, 16, kLinear, true>();
-  conv_attr<KN, 32, 16, kAccum, true>();
-  conv_attr<KN, 32, 16, kTauSplit, true>();
-  conv_attr<KN, 16, 32, kAccum>();
-  conv_attr<KN, 32, 32, kAccum>();
-  conv_attr<KN, 32, 16, kAccum>();
+  conv_split_attr<KN, 16, 32, kGeluSplit, true>();
+  conv_split_attr<KN, 32, 32, kGeluSplit, true>();
+  conv_split_attr<KN, 32, 16, kTauSplit, true>();
+  conv_split_attr<KN, 16, 32, kAccum, false>();
+  conv_split_attr<KN, 32, 32, kAccum, false>();
+  conv_split_attr<KN, 32, 16, kAccum, false>();
 }
 
 void cnn_init() {
