@@ -591,13 +591,15 @@ __global__ void k_band_forcing(const PackArgs a, double eps, double* A) {
   }
 }
 
-template <typename R>
-__global__ void k_spectral_energy(const PackArgs a, int K1, int K2, int compact, double kfac, int weight_k2,
+// NC fields of a kind known at compile time, two modes a trip: the loads of all of
+// them are in flight together (a loop over the fields: 76 us at 256^3 FP32)
+template <typename R, int NC>
+__global__ void __launch_bounds__(256) k_spectral_energy(const PackArgs a, int K1, int K2, int compact, double kfac, int weight_k2,
                                   double* out, int mask23) {
   using C = typename V2<R>::T;
   const unsigned nm = unsigned(K1) * K2 * (a.D == 3 ? K2 : 1);  // < 2^31 at every size
   double e = 0;
-#pragma unroll 4
+#pragma unroll 2
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nm; i += gridDim.x * blockDim.x) {
     const unsigned r = i / K1;
     const int ix = int(i - r * K1);
@@ -616,11 +618,12 @@ __global__ void k_spectral_energy(const PackArgs a, int K1, int K2, int compact,
       if (weight_k2) w *= kfac * kfac * double(ix * ix + iky * iky + ikz * ikz);
       if (mask23 && (ix > a.kc || iky > a.kc || -iky > a.kc || ikz > a.kc || -ikz > a.kc)) w = 0.0;
     }
+    C v[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = __ldg(static_cast<const C*>(a.src[c]) + i);
     double s = 0;
-    for (int c = 0; c < a.ncomp; ++c) {
-      const C v = static_cast<const C*>(a.src[c])[i];
-      s += double(v.x) * double(v.x) + double(v.y) * double(v.y);
-    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) s += double(v[c].x) * double(v[c].x) + double(v[c].y) * double(v[c].y);
     e += w * s;
   }
   e = block_sum(e);
@@ -1007,7 +1010,8 @@ template <typename R> void launch_spectral_energy(const void* const* u, int ncom
   long long nb = (nm + 255) / 256;
   if (nb > 148 * 8) nb = 148 * 8;
   if (nb < 1) nb = 1;
-  k_spectral_energy<R><<<unsigned(nb), 256, 0, st>>>(a, K1, K2, compact, kfac, weight_k2, out, mask23);
+  if (ncomp == 2) k_spectral_energy<R, 2><<<unsigned(nb), 256, 0, st>>>(a, K1, K2, compact, kfac, weight_k2, out, mask23);
+  else k_spectral_energy<R, 3><<<unsigned(nb), 256, 0, st>>>(a, K1, K2, compact, kfac, weight_k2, out, mask23);
 }
 
 // ---------------------------------------------------------------------------
