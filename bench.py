@@ -524,7 +524,7 @@ def les_adjoint_measure(dev, nsteps, ck, plain_instances=2):
     Delta/h = 4), CNN closure, nsteps-step RK4 rollout checkpointed every ck
     steps, trajectory-MSE loss against a target rollout of the perturbed closure
     (weights x (1 + 0.01 N(0,1))), gradient by the hand-written adjoint.
-    Batched: FP32 with the tensor-core CNN in split precision (three passes
+    Batched: FP32 with the tensor-core CNN in split precision (three products
     over hi/lo operand parts per convolution, FP32 accumulate), the 8 jobs
     concurrently (sc_rollout_adjoint_batch); beside it the same with one BF16
     pass per convolution (the adjoint takes the BF16 roundings as identities)
@@ -583,7 +583,7 @@ def les_adjoint_measure(dev, nsteps, ck, plain_instances=2):
         return res, t
 
     res32, t_batch = run_batch(True)
-    # the tensor-core CNN in split precision (three passes over hi/lo parts per convolution)
+    # the tensor-core CNN in split precision (three products of hi/lo parts per convolution)
     res_sp, t_batch_sp = run_batch(True, split=True)
     # the CUDA-core FP32 closure: 4 of the 8 jobs, one timed batch (about a minute)
     ncc = 4
@@ -609,8 +609,8 @@ def les_adjoint_measure(dev, nsteps, ck, plain_instances=2):
     return {
         "metric": "batched LES+adjoint steps/s (8 x 64^3 training rollouts: forward, loss and adjoint per step)",
         "what": "the 8 jobs batched on the tensor cores in split precision (SC_CLOPT_CNN_SPLIT): each convolution "
-                "three tcgen05 passes A_hi W_hi + A_lo W_hi + A_hi W_lo over FP16 (forward) or BF16 (input "
-                "gradient) hi/lo operand parts, FP32 accumulation, GELU with tanhf; weight gradients on CUDA cores",
+                "the tcgen05 products A_hi W_hi + A_lo W_hi + A_hi W_lo over FP16 (forward) or BF16 (input "
+                "gradient) hi/lo operand parts, FP32 accumulation, GELU with tanhf; weight gradients on tcgen05 too",
         "value": 8 * nsteps / t_batch_sp, "unit": "steps/s", "s_per_training_step": t_batch_sp,
         "plain_fp64_steps_per_s": nsteps / t_plain, "plain_fp64_s_per_instance": t_plain,
         "speedup_vs_plain": (8 * t_plain) / t_batch_sp,
@@ -633,7 +633,7 @@ def les_adjoint_measure(dev, nsteps, ck, plain_instances=2):
             "grad_rel_err_fp32_vs_fp64": errs_cc},
         "config": f"64^3, nu in {list(ADJ_NU)}, Delta/h={ADJ_DH}, RK4 dt={ADJ_DT}, {nsteps} steps, checkpoint every "
                   f"{ck}; CNN closure (4 layers 3x3x3, 32 channels, GELU, seeded Kaiming weights): batched on "
-                  "tcgen05 (forward and input-gradient convolutions; weight gradients on CUDA cores in FP32), "
+                  "tcgen05 (forward and input-gradient convolutions and weight gradients), "
                   "plain on CUDA cores in FP64 one instance after another; target rollout of the closure with "
                   "weights x (1 + 0.01 N(0,1)); initial fields sfs! of seeded 128^3 fields; gradient errors of the "
                   f"first {plain_instances} jobs against the plain FP64 path's; host wall clock around the "

@@ -24,8 +24,9 @@
 // the tensor memory is freed always keeps the full default bound.
 //
 // Split precision (SC_CLOPT_CNN_SPLIT): each operand is stored as two 16-bit
-// parts x = hi + lo, and a convolution is three launches of the same kernel,
-// A_hi W_hi + A_lo W_hi + A_hi W_lo, accumulated in an FP32 channels-last
+// parts x = hi + lo, and a convolution is A_hi W_hi + A_lo W_hi + A_hi W_lo: one
+// fused launch where the operands fit shared memory, else three launches of the
+// same kernel accumulated in an FP32 channels-last
 // buffer by the epilogue modes kLinear, kAccum and a last mode that applies
 // bias and GELU (tanhf) and writes the hi/lo activations (or tau).  Forward
 // passes use FP16 parts (kind::f16 with both operands f16); the adjoint's
@@ -770,7 +771,7 @@ template <int KN> static void cnn_forward_n(const CnnArgs& a, cudaStream_t st) {
   conv_launch<KN, 32, 16, kTau>(grid, a3, a.w[3], a.b[3], o4, a.err, a.wait_limit, st);
 }
 
-// split precision: FP16 hi/lo inputs and weights, three passes per layer,
+// split precision: FP16 hi/lo inputs and weights, three products per layer,
 // exact GELU; layer l accumulates in pre[l] when given (the adjoint keeps h
 // there), else in acc; layer 4 always in acc
 template <int KN> static void cnn_forward_split_n(const CnnArgs& a, cudaStream_t st) {
@@ -845,7 +846,7 @@ template <int KN> static void cnn_backward_n(const CnnBwdArgs& a, cudaStream_t s
   k_gin_planar<<<nblk(npts), 256, 0, st>>>(a.gf, a.gin_planar, npts);
 }
 
-// split precision: BF16 hi/lo gradients and transposed weights (three passes
+// split precision: BF16 hi/lo gradients and transposed weights (three products
 // per input-gradient convolution), weight gradients from the hi + lo sums
 template <int KN> static void cnn_backward_split_n(const CnnBwdArgs& a, cudaStream_t st) {
   const long long npts = (long long)KN * KN * KN;

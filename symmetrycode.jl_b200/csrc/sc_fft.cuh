@@ -1,7 +1,8 @@
-// Mixed-radix (2, 3, 5) FFT engine for a tile of pencils held in shared memory.
+// Register DFTs of radix 2 to 45, and the mixed-radix (2, 3, 5) FFT engine for a
+// tile of pencils held in shared memory (sizes below 32).
 //
-// Every spectral transform of the solver (the cuFFT/FFTW `plan_rfft` calls of
-// src/solver.jl:210-215,432-453 in the reference) is built from this engine: a
+// The spectral transforms of the solver stand in for the cuFFT/FFTW `plan_rfft`
+// calls of src/solver.jl:210-215,432-453 in the reference.  In the engine a
 // CTA loads a tile of NPEN pencils of length N into shared memory, runs the
 // passes of a Stockham autosort FFT with radices from {2..16} drawn from
 // N = 2^a 3^b 5^c, and writes the tile back.  Each pass reads the R inputs of

@@ -146,7 +146,7 @@ template <typename R> void launch_spectral_energy(const void* const* u, int ncom
                                                   double kfac, int weight_k2, double* out,
                                                   cudaStream_t st, int mask23 = 0);
 bool fft_size_supported(int n);
-// two-level FP32 engine (sc_fast.cu) for N in {64, 128, 256, 810}
+// FP32 sizes whose column sweeps have variants (sc_fast.cu): 64, 128, 256, 810
 bool fast_supported(int N);
 bool init_fast(int N);
 bool launch_col2(int N, bool inv, const ColArgs& a, const void* tw, cudaStream_t st);

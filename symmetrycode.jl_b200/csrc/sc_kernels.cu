@@ -4,12 +4,17 @@
 // which runs `nonlinearity!` src/solver.jl:434-456, `viscosity!` :458-476 and
 // `tensordivergence!` :509-521 around 9 cuFFT calls) is five sweeps over HBM:
 //
-//   k_col_inv   z: compact 2/3 cube (kx, ky, kz)  -> (kx, ky, z)     3 comps
-//   k_col_inv   y: (kx, ky, z)                    -> (kx, y, z)      3 comps
-//   k_xsweep_ns x: c2r, u_i u_j / n^D, r2c        -> (kx, y, z)      6 comps
-//   k_col_fwd   y: (kx, y, z)                     -> (kx, ky, z)     6 comps
-//   k_col_fwd   z: (kx, ky, z)                    -> (kx, ky, kz)    6 comps
-//   k_epilogue     viscous term, divergence, projection, forcing, RK update
+//   inverse z  compact 2/3 cube (kx, ky, kz)  -> (kx, ky, z)     3 comps
+//   inverse y  (kx, ky, z)                    -> (kx, y, z)      3 comps
+//   x          c2r, u_i u_j / n^D, r2c        -> (kx, y, z)      6 comps
+//   forward y  (kx, y, z)                     -> (kx, ky, z)     6 comps
+//   forward z  (kx, ky, z)                    -> (kx, ky, kz)    6 comps
+//   epilogue   viscous term, divergence, projection, forcing, RK update
+//
+// This file holds the dispatch, the sweeps of the sizes below 32 on the
+// shared-memory engine (sc_fft.cuh), the spectral point kernels and the FP64
+// reductions; sizes from 32 on take the register sweeps (sc_col.cuh, sc_xrow.cuh,
+// sc_fast.cu).
 //
 // Only the modes kept by the 2/3 rule (|k_i| <= n/3) are ever stored, so the
 // zero modes `twothirds!` (src/solver.jl:371-389) would mask are never read.
