@@ -15,14 +15,14 @@
 // I2 leaves every lane with exactly the points its F1 needs, so the products
 // are formed in registers.  A warp holds W = 32 / N1 row pairs, so every
 // exchange is inside one warp: __syncwarp only, no CTA barrier, and the CTAs
-// are just bundles of independent warps.  Slots have odd row strides (SP, SQ),
-// which makes both sides of every exchange free of bank conflicts, and the
-// twiddles come from tables in the order the lanes read them.
+// are just bundles of independent warps.  The slots' row strides (SP, SQ) make
+// both sides of every exchange, and the gather of S, nearly free of bank conflicts;
+// the twiddles come from tables in the order the lanes read them.
 //
 // What bounds it: FP32 issue (FP64: the FP64 pipe) at large N with the rows
 // streaming from HBM.  Against the CTA-wide kernels it replaces it moves about
 // half the shared-memory bytes (47 -> 26 KB a row at N = 256, FP32): 2 GB of rows at
-// N = 256 1069 -> 616 us in FP32 and 2687 -> 570 in FP64, at 540 in FP64 1867 -> 905.
+// N = 256 1069 -> 603 us in FP32 and 2687 -> 570 in FP64, at 540 in FP64 1867 -> 905.
 #pragma once
 #include "sc_fft.cuh"
 #include "sc_internal.h"
@@ -35,9 +35,20 @@ template <typename R, int N> struct XRowCfg {
   using C = typename V2<R>::T;
   static constexpr int N1 = XSplit<R, N>::N1, N2 = XSplit<R, N>::N2;
   static constexpr int W = 32 / N1;               // row pairs per warp
-  static constexpr int SP = N2 | 1, SQ = N1 | 1;  // slot row strides of the inverse / forward exchange
+  // Slot row strides of the inverse / forward exchange.  Odd ones keep both sides
+  // of an exchange free of bank conflicts; S reads 16 / N2 neighbouring values of
+  // m for each k' at once, so in FP32 (16 lanes a phase) with N2 = 8 or 4 the
+  // forward stride is 2 or 4 times an odd number, and the slot stride odd: k' SQ + m
+  // and, over neighbouring pencils, k' SQ + q PS are then distinct modulo 16.
+  // Against odd strides everywhere, product sweep of 2 GB of rows, FP32: N = 64 590
+  // -> 492 us, 60 564 -> 503, 128 577 -> 564, 256 616 -> 603; 160 to 240 equal.
+  static constexpr bool P8 = sizeof(R) == 4 && N2 == 8, P4 = sizeof(R) == 4 && N2 == 4;
+  static constexpr int SP = N2 | 1;
+  static constexpr int SQ = P8 ? (N1 + 1) / 4 * 4 + 2 : P4 ? (N1 + 3) / 8 * 8 + 4 : N1 | 1;
   static constexpr int PSM = N1 * SP > N2 * SQ ? N1 * SP : N2 * SQ;
-  static constexpr int PS = (PSM + 7) / 16 * 16 + 8;  // = 8 (mod 16): two groups of 8 lanes meet no bank twice
+  static constexpr int PO = P8 ? 9 : P4 ? 5 : 8;  // = 8 (mod 16) else: two groups of 8 lanes meet no bank twice
+  static constexpr int PS = (PSM + 15 - PO) / 16 * 16 + PO;
+  static_assert(SQ >= N1 && PS >= PSM, "slot strides");
   static constexpr int KC = N / 3;
   static constexpr size_t slots(int n) { return size_t(n) * W * PS * sizeof(C); }
   // warps per CTA and CTAs per SM for n slots a warp: as many warps as shared
@@ -214,11 +225,11 @@ k_xr_ns(const __grid_constant__ XArgs a, const typename V2<R>::T* __restrict__ t
   const C* in2 = static_cast<const C*>(a.in[D == 3 ? 2 : 1]);
 #pragma unroll 1
   for (int it = lane; it < W * NI * N2; it += 32) {
-    const int w = it / (NI * N2), p = (it / N2) % NI, j = it % N2;
+    const int q = it / N2, j = it - q * N2, p = q / W, w = q - p * W;  // slot q: pencil p of row pair w
     const int row = 2 * (rp0 + w);
     const C* ra = (p < 2 ? in0 : in2) + (row + (p == 1)) * K1i;
     const C* rb = p < 2 ? in1 + (row + p) * K1i : in2 + (row + 1) * K1i;
-    C* slot = sm + (p * W + w) * PS;
+    C* slot = sm + q * PS;
     if constexpr (WIDE) xr_i1_wide<R, N>(ra, rb, K1i - 1, rp0 + w < npair, j, t1, slot);
     else xr_i1<R, N, KC>(ra, rb, rp0 + w < npair, j, t1, slot);
   }
@@ -569,11 +580,11 @@ k_xr_vmax(const __grid_constant__ XPlainArgs a, const typename V2<R>::T* __restr
   const C* in2 = static_cast<const C*>(a.in[D == 3 ? 2 : 1]);
 #pragma unroll 1
   for (int it = lane; it < W * D * N2; it += 32) {
-    const int w = it / (D * N2), p = (it / N2) % D, j = it % N2;
+    const int q = it / N2, j = it - q * N2, p = q / W, w = q - p * W;
     const int row = 2 * (rp0 + w);
     const C* ra = (p < 2 ? in0 : in2) + (row + (p == 1)) * (KC + 1);
     const C* rb = p < 2 ? in1 + (row + p) * (KC + 1) : in2 + (row + 1) * (KC + 1);
-    xr_i1<R, N, KC>(ra, rb, rp0 + w < npair, j, t1, sm + (p * W + w) * PS);
+    xr_i1<R, N, KC>(ra, rb, rp0 + w < npair, j, t1, sm + q * PS);
   }
   __syncwarp();
   const int w = lane / N1, i = lane - w * N1;
