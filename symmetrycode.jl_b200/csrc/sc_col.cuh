@@ -20,7 +20,7 @@ namespace sc {
 // T consecutive kx per tile; S = 1 transposes the split (N2 first)
 template <typename R, int N, int T, int S = 0> struct Col2Cfg {
   using C = typename V2<R>::T;
-  static constexpr int N1 = S ? CSplit<N>::N2 : CSplit<N>::N1, N2 = S ? CSplit<N>::N1 : CSplit<N>::N2;
+  static constexpr int N1 = S ? CSplit<R, N>::N2 : CSplit<R, N>::N1, N2 = S ? CSplit<R, N>::N1 : CSplit<R, N>::N2;
   static constexpr int NJ = N1 > N2 ? N1 : N2;
   static constexpr int NT = T * NJ;
   static constexpr int SR = N2 * T + 8;  // exchange row stride (+8: half-bank shift between rows)
