@@ -22,6 +22,7 @@ import oracle as O
 import symcode as S
 from _util import rel_l2, to_dev, to_np
 from oracle import triad as T
+from test_gpu_les import KINDS, _models
 
 pytestmark = pytest.mark.gpu
 
@@ -117,3 +118,54 @@ def test_sfs_on_the_reduced_grid_matches_the_oracle(n, m, dtype, captured):
     s1 = [O.twothirds(O.gaussianfilter(O.cutoff(c, od, ol), d, ol), ol) for c in O.nonlinearity(u, od)]
     scale = math.sqrt(sum(float(np.sum(np.abs(c) ** 2)) for c in s1))
     assert math.sqrt(sum(float(np.sum(np.abs(to_np(x) - y) ** 2)) for x, y in zip(tau, rt))) < tol * scale
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("D,n,dtype", ((3, 32, torch.float64), (3, 36, torch.float32), (3, 60, torch.float64),
+                                       (3, 64, torch.float32), (3, 72, torch.float64), (3, 90, torch.float32),
+                                       (3, 96, torch.float64), (3, 128, torch.float32), (2, 90, torch.float32),
+                                       (2, 160, torch.float64)))
+def test_closure_sweeps_match_the_oracle(kind, D, n, dtype):
+    """The closures' point functions inside the x sweep and the test filter inside
+    the z sweep.  A right-hand side, so the tolerances of one."""
+    if kind == "verstappen" and D == 2:
+        pytest.skip("Q-R model is only defined in 3D")
+    g, go = S.Grid(D, n, dtype=dtype, device="cuda:0"), O.Grid(D, n)
+    u = O.random_field(go, seed=21, kpeak=3)
+    delta = 2 * go.l / n
+    cl, model = _models(kind, delta, g, D)
+    ref = [O.twothirds(c, go) for c in O.les_rhs(u, go, lambda uu, GG: model(uu, GG, go), 1e-3)]
+    du = S.vectorfield(g)
+    S.les_(du, [to_dev(c, g) for c in u], g, cl, 1e-3)
+    assert rel_l2([to_np(c) for c in du], ref) < (1e-12 if dtype == torch.float64 else 1e-5)
+
+
+def test_split_training_gradient_at_128():
+    """Forward passes, input gradients and weight gradients of the tensor-core
+    network at its larger size against FP64.  Tolerance of the 64^3 case in
+    test_gpu_adjoint.py: one step with weights 100 % off leaves a misfit of the
+    size that its 40 steps with 1 % do, so the FP32 rounding of the states weighs
+    the same."""
+    n, dt, nu = 128, 2.5e-3, 1e-3
+    go = O.Grid(3, n)
+    u = O.random_field(go, seed=7, kpeak=4)
+    ws, bs = S.kaiming_cnn_weights(5)
+    theta = S.pack_cnn_params(ws, bs)
+    off = theta * (1 + np.random.default_rng(8).standard_normal(theta.size))
+    res = []
+    for dtype in DTYPES:
+        g = S.Grid(3, n, dtype=dtype, device="cuda:0")
+        if dtype == torch.float32:
+            cl = S.create_cnn_closure(4 * go.l / n, nu, g, ws, bs, mu=5.0, sigma=2.0, split=True)
+        else:
+            cl = S.create_cnn_fp_closure(4 * go.l / n, nu, g, ws, bs, mu=5.0, sigma=2.0)
+        u0 = [to_dev(c, g) for c in u]
+        S.closure_set_params(cl, off)
+        traj = S.rollout_record(g, cl, u0, dt, nu, 1)
+        S.closure_set_params(cl, theta)
+        res.append(S.rollout_adjoint(g, cl, u0, traj, dt, nu, 1, ckpt_every=1))
+        cl.close()
+        g.close()
+    (l32, g32), (l64, g64) = res
+    assert abs(l32 - l64) < 1e-4 * l64
+    assert np.linalg.norm(g32 - g64) < 1e-4 * np.linalg.norm(g64)
