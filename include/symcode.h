@@ -398,7 +398,11 @@ SC_API int sc_rollout_adjoint_batch(int njobs, const sc_rollout_job* jobs, int* 
  * u_hat: DNS full layout (D pointers).  ubar_hat: ndelta*D LES full-layout
  * fields (d-major); tau_hat: ndelta*(3|6) LES full-layout fields, pair order
  * xx, yy[, zz], xy[, yz, zx].  The two plans must be distinct, same D, l,
- * precision and device, n_les <= n_dns. */
+ * precision and device, n_les <= n_dns.  Asynchronous.  The products may be
+ * formed on fewer points than n_dns (as many as the kept modes need); the DNS
+ * plan's first call for such a size fills a table of a few KB on the host and
+ * waits for its copy, not for the work queued on `stream`.  A first call under
+ * stream capture forms the products on the DNS grid instead. */
 SC_API int sc_filter_sfs(sc_plan* dns, sc_plan* les, const void* const* u_hat, const double* deltas, int ndelta,
                          void* const* ubar_hat, void* const* tau_hat, void* stream);
 /* filter_reynolds(ubar, g, visc, Delta) (src/solver.jl:768-774):

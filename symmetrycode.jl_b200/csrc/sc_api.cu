@@ -74,8 +74,11 @@ struct sc_plan {
   double* shells = nullptr;  // kc + 3 shell sums of the spectrum and the diagnostics
   int* err = nullptr;       // device word set when a bounded wait of a TMA-fed sweep ran out
   void* fa = nullptr, *fb = nullptr;  // full-spectrum scratch (lazy)
-  void* twr = nullptr;                // twiddle buffer of the filter's reduced grid
-  int nr = 0;                         // its size (0: not filled yet)
+  // The filter's reduced grids (reduced_grid): one twiddle buffer per size the
+  // plan can meet, written once and never again, so that kernels in flight or in
+  // a caller's graph keep theirs.
+  struct Reduced { int m; void* tw; bool filled; };
+  std::vector<Reduced> reduced;
   std::vector<void*> allocs;
   cudaStream_t cap = nullptr;
   cudaGraphExec_t g_rk4 = nullptr;
@@ -187,18 +190,40 @@ int plan_alloc(sc_plan* p, void** out, size_t bytes) {
   return SC_OK;
 }
 
+// The grid on which the DNS products of the filter are formed.  Only the modes
+// |k_i| <= kout of the products are kept, and the inputs have |k_i| <= kc, so any
+// M > 2 kc + kout points per axis give those modes free of aliasing, as the DNS
+// grid does: 810 -> 640 for 128-point LES data, half the rows and points of every
+// sweep.  Taken when at least a tenth of the points per axis go (256 -> 128 would
+// leave 240: no faster, and a radix-5 size rounds a little more than a power of
+// two).  0: the DNS grid, also where the x sweep does not take the shape.
+int reduced_grid(const sc_plan* p, int kout) {
+  const int m = sc::sweep_size_from(2 * p->kc + kout + 1);
+  return p->D == 3 && m > 0 && 10 * m <= 9 * p->n && p->kc > m / 3 && kout <= m / 5 ? m : 0;
+}
+
 // The plan's small buffers in one allocation (each costs a fraction of a
-// millisecond): twiddles, those of a smaller size (810's own tables included),
-// scalars, shell sums, the error word.
+// millisecond): twiddles, those of the filter's reduced grids (three sizes at
+// most), scalars, shell sums, the error word.
 int plan_tables(sc_plan* p) {
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t tw = up(sc::twiddle_buffer_bytes(p->n, p->esz));
-  const size_t twr = p->D == 3 ? up(3 * (size_t)p->n * p->esz + sc::xpair810_twiddle_bytes() + sc::X4Tab::SIZE * 8) : 0;
+  size_t twr = 0;
+  for (int k = 1; k <= p->kc; ++k) {
+    const int m = reduced_grid(p, k);  // grows with k
+    if (!m || (!p->reduced.empty() && p->reduced.back().m == m)) continue;
+    p->reduced.push_back({m, nullptr, false});
+    twr += up(sc::twiddle_buffer_bytes(m, p->esz));
+  }
   const size_t shells = up((p->kc + 3) * sizeof(double));
   const int rc = plan_alloc(p, &p->tw, tw + twr + shells + 512);
   if (rc) return rc;
   char* b = static_cast<char*>(p->tw) + tw;
-  if (twr) p->twr = b;
+  size_t off = 0;
+  for (auto& r : p->reduced) {
+    r.tw = b + off;
+    off += up(sc::twiddle_buffer_bytes(r.m, p->esz));
+  }
   p->shells = reinterpret_cast<double*>(b + twr);
   p->dscal = reinterpret_cast<double*>(b + twr + shells);
   p->err = reinterpret_cast<int*>(b + twr + shells + 256);
@@ -1088,61 +1113,66 @@ int energy_impl(sc_plan* p, const void* const* u, int compact, int weight_k2, do
   return SC_OK;
 }
 
-// The grid on which the DNS products of the filter are formed.  Only the modes
-// |k_i| <= kout of the products are kept, and the inputs have |k_i| <= kc, so any
-// M > 2 kc + kout points per axis give those modes free of aliasing, as the DNS
-// grid does: 810 -> 640 for 128-point LES data, half the rows and points of every
-// sweep.  Taken when at least a tenth of the points per axis go (256 -> 128 would
-// leave 240: no faster, and a radix-5 size rounds a little more than a power of
-// two).  0: the DNS grid, also where the x sweep does not take the shape.
-int reduced_grid(const sc_plan* p, int kout) {
-  const int m = sc::sweep_size_from(2 * p->kc + kout + 1);
-  return p->D == 3 && m > 0 && 10 * m <= 9 * p->n && p->kc > m / 3 && kout <= m / 5 ? m : 0;
-}
-
-// Fills the plan's second twiddle buffer for size m (once per size).  Not while
-// the stream is being captured: false then, and the caller takes the DNS grid.
+// The twiddle buffer of the reduced grid of m points in *tw, filled on first use
+// by a copy on the plan's own stream: the call waits for that copy, not for the
+// work queued on `st`.  nullptr while `st` is being captured and the buffer is
+// not filled yet: the caller then takes the DNS grid.
 template <typename R>
-bool reduced_twiddles(sc_plan* p, int m, cudaStream_t st) {
-  if (p->nr == m) return true;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
-  if (!sc::init_kernels<R>(m)) return false;
-  const std::vector<unsigned char> img = twiddle_image<R>(m);
-  p->nr = 0;
-  if (cudaMemcpyAsync(p->twr, img.data(), img.size(), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return false;
-  p->nr = m;
-  return true;
+int reduced_twiddles(sc_plan* p, int m, cudaStream_t st, const void** tw) {
+  *tw = nullptr;
+  sc_plan::Reduced* r = nullptr;
+  for (auto& q : p->reduced)
+    if (q.m == m) r = &q;
+  if (!r) return SC_OK;
+  if (!r->filled) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cudaGetLastError();  // the launches report it
+    else if (cs == cudaStreamCaptureStatusNone) {
+      // another thread may be capturing meanwhile
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      const std::vector<unsigned char> img = twiddle_image<R>(m);
+      cudaError_t e = sc::init_kernels<R>(m) ? cudaSuccess : cudaErrorUnknown;
+      if (e == cudaSuccess) e = cudaMemcpyAsync(r->tw, img.data(), img.size(), cudaMemcpyHostToDevice, p->cap);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(p->cap);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(SC_ERR_CUDA, "twiddles of %d points: %s", m, cudaGetErrorString(e));
+      }
+      r->filled = true;
+    }
+  }
+  if (r->filled) *tw = r->tw;
+  return SC_OK;
 }
 
 // compact u -> F[u_i u_j]/n^D on the compact cube of half-width kout, formed on m points per axis
 template <typename R>
-int products_reduced(sc_plan* p, void* const* u, int kout, int m, void* const* sig, cudaStream_t st) {
+int products_reduced(sc_plan* p, void* const* u, int kout, int m, const void* tw, void* const* sig, cudaStream_t st) {
   const int K1 = p->K1, kc = p->kc, K1o = kout + 1, ld = even_up(K1), ldo = even_up(K1o);
   sc::ColArgs a = z_inverse_args(K1, p->K2, m, kc, ld);
   for (int c = 0; c < 3; ++c) { a.in[c] = u[c]; a.out[c] = p->be[c]; }
   a.ncomp = 3;
-  sc::launch_col_inv<R>(m, a, p->twr, st);
+  sc::launch_col_inv<R>(m, a, tw, st);
   sc::ColArgs b = y_inverse_args(K1, m, kc, ld);
   for (int c = 0; c < 3; ++c) { b.in[c] = p->be[c]; b.out[c] = p->cc[c]; }
   b.ncomp = 3;
-  sc::launch_col_inv<R>(m, b, p->twr, st);
+  sc::launch_col_inv<R>(m, b, tw, st);
   sc::XArgs x{};
   for (int c = 0; c < 3; ++c) x.in[c] = p->cc[c];
   for (int c = 0; c < 6; ++c) x.out[c] = p->dd[c];
   x.D = 3; x.K1in = K1; x.K1out = K1o; x.nrows = (long long)m * m; x.scale = 1.0 / ((double)m * m * m);
   x.ldo = ldo;
-  if (!sc::launch_xsweep_ns<R>(m, x, p->twr, st)) return fail(SC_ERR_SIZE, "no product sweep on %d points", m);
+  if (!sc::launch_xsweep_ns<R>(m, x, tw, st)) return fail(SC_ERR_SIZE, "no product sweep on %d points", m);
   sc::ColArgs f = y_forward_args(K1o, m, kout, ldo);
   for (int c = 0; c < 6; ++c) { f.in[c] = p->dd[c]; f.out[c] = p->be[c]; }
   f.ncomp = 6;
-  sc::launch_col_fwd<R>(m, f, p->twr, st);
+  sc::launch_col_fwd<R>(m, f, tw, st);
   sc::ColArgs g = z_forward_args(K1o, m, kout, ldo);
   for (int c = 0; c < 6; ++c) { g.in[c] = p->be[c]; g.out[c] = sig[c]; }
   g.ncomp = 6;
-  sc::launch_col_fwd<R>(m, g, p->twr, st);
+  sc::launch_col_fwd<R>(m, g, tw, st);
   return check_launch("product pipeline");
 }
 
@@ -1153,7 +1183,9 @@ int filter_impl(sc_plan* dns, sc_plan* les, const void* const* u, const double* 
   int rc = pack_state<R>(dns, u, dns->S, st);
   if (rc) return rc;
   const int m = reduced_grid(dns, les->kc);
-  if (m && reduced_twiddles<R>(dns, m, st)) rc = products_reduced<R>(dns, dns->S, les->kc, m, dns->sig, st);
+  const void* twr = nullptr;
+  if (m && (rc = reduced_twiddles<R>(dns, m, st, &twr))) return rc;
+  if (twr) rc = products_reduced<R>(dns, dns->S, les->kc, m, twr, dns->sig, st);
   else rc = products<R>(dns, dns->S, st, nullptr, les->kc, dns->sig);
   if (rc) return rc;
   for (int d = 0; d < nd; ++d) {
