@@ -360,7 +360,9 @@ SC_API int sc_plan_status(sc_plan* plan, int* status);
  * of the LES right-hand side (FFT transposes, product and viscous terms,
  * projection, the CNN's convolutions and GELUs and its Re_Delta channel),
  * recomputing the states from checkpoints every `ckpt_every` steps.
- * All three are synchronous. */
+ * All three are synchronous; they return SC_ERR_TIMEOUT, with results that are
+ * not to be used, once a bounded wait of the closure's kernels has run out
+ * (SC_OPT_WAIT_LIMIT). */
 SC_API size_t sc_rollout_traj_bytes(const sc_plan* plan, int nsteps);
 SC_API int sc_rollout_record(sc_plan* plan, sc_closure* closure, const void* const* u0, double dt, double visc,
                              int nsteps, void* traj, void* stream);

@@ -2545,13 +2545,17 @@ int rollout_impl(sc_plan* p, sc_closure* cl, const void* const* u0, const void* 
     }
   }
   double h = 0;
+  int timeout = 0;
   if (!rc) {
+    if (cl && cl->err) SC_CU_FREE(cudaMemcpyAsync(&timeout, cl->err, sizeof(int), cudaMemcpyDeviceToHost, st));
     SC_CU_FREE(cudaMemcpyAsync(&h, B.dloss, sizeof(double), cudaMemcpyDeviceToHost, st));
     if (adj && cl && cl->gw) SC_CU_FREE(cudaMemcpyAsync(grad, cl->gw, cl->nparam * sizeof(double), cudaMemcpyDeviceToHost, st));
   }
   freeall();
   SC_CU(cudaStreamSynchronize(st));
   if (loss) *loss = traj ? h / nsteps : 0.0;
+  // a kernel that gave up has left out its share of the stress or of the gradient
+  if (timeout) return fail(SC_ERR_TIMEOUT, "a bounded wait of the CNN kernels ran out");
   return rc;
 }
 #undef SC_CU_FREE
