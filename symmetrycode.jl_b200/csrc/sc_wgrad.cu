@@ -20,15 +20,21 @@
 // of valid rows; the other rows multiply whatever follows in shared memory and
 // are never read.
 //
-// The tensor core does not round its FP32 accumulations to nearest: over a CTA's
-// thousand of them the gradient was off by 1.7e-5 where the FP32 kernel's was off
-// by 4.2e-6.  So every block starts from zero (48 accumulations) and eight warps
-// add its result to FP32 sums in registers.
+// The tensor core truncates its FP32 accumulations: over a CTA's thousand of them
+// the gradient was off by 1.7e-5 where the FP32 kernel's was off by 4.2e-6.  So
+// every half block starts from zero (8 accumulations of a size with the sum) and
+// eight warps add its result to FP32 sums in registers.  What truncation has then
+// taken from a result is within 20 % one part in 2^23 of it, whatever the data
+// (white 1.0e-7 to 1.1e-7, smooth 1.0e-7 to 1.2e-7; all terms of one sign 1.6e-7),
+// so the addition gives it back as an FMA with 1 + 2^-23.  Against FP64, 64^3,
+// 32 -> 32, split, white | smooth data: read out once a block 2.7e-7 | 2.3e-7, the
+// FP32 kernel 4.1e-7 | 2.4e-8.
 //
 // A block is 4 output rows of 64 voxels: 4 g rows and 6 input rows, staged by
 // seven warps in one of two buffers while the MMA thread works on the other.
-// What bounds it: the MMA rate at N = 96 (about 69 cycles an MMA) and M half
-// used.  64^3, 32 -> 32, split: 963 us on CUDA cores before.
+// What bounds it: the MMAs, about 88 cycles each whatever their N, and M half
+// used.  64^3, 32 -> 32, split: 160 us read out once a block, 165 us twice, 963 us
+// on CUDA cores.
 #include <cuda_fp16.h>
 
 #include "sc_tcgen05.cuh"
@@ -42,6 +48,7 @@ namespace {
 // that warp 2 issues the MMAs
 constexpr int kThreads = 512, kStage = 7 * 32, kMmaWarp = 2;
 constexpr int TX = 64, YB = 4;         // voxels of a row tile, output rows of a block
+constexpr int SB = 2, NSB = YB / SB;   // output rows, read-outs of a block
 constexpr int PLANE = (TX + 2) * 16;   // bytes of 8 channels of a row with its x halo
 // 16-byte x 8 stores of consecutive threads fall on distinct banks: PLANE = 32 (mod 128)
 static_assert(PLANE % 128 == 32, "plane stride");
@@ -80,7 +87,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad_tc(const WgradArgs p) {
   extern __shared__ __align__(128) unsigned char sm[];
   uint64_t* full = reinterpret_cast<uint64_t*>(sm + Cfg::SMEM - 128);  // [2] staged by all staging threads
   uint64_t* done = full + 2;                                            // [2] MMAs of the buffer's block complete
-  uint64_t* drained = done + 2;                                         // accumulators of a block read out
+  uint64_t* summed = done + 2;                                          // MMAs of SB rows complete
+  uint64_t* drained = summed + 1;                                       // accumulators of SB rows read out
   uint32_t* tslot = reinterpret_cast<uint32_t*>(drained + 1);
   int* abort_flag = reinterpret_cast<int*>(tslot + 1);
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
@@ -95,6 +103,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad_tc(const WgradArgs p) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(full + q)), "r"(kStage));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(done + q)));
     }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(summed)));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(smem_u32(drained)));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *abort_flag = 0;
@@ -122,7 +131,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad_tc(const WgradArgs p) {
   constexpr int NCOL = Cfg::NCOL, NCH = (NCOL / 16 + 3) / 4;  // 16-column chunks of a reader warp
   float acc[NCH][16] = {};
   if (stager) {
-    const int gc = sid % CO;  // this thread's channel chunk of g (256 is a multiple of CO)
+    static_assert(kStage % CO == 0, "a staging thread keeps its channel chunk of g");
+    const int gc = sid % CO;
     for (int b = b0; b < b1 && ok; ++b) {
       const int i = b - b0, buf = i & 1;
       unsigned char* sg = sm + buf * Cfg::BUF;
@@ -190,9 +200,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad_tc(const WgradArgs p) {
     }
   } else if (reader) {
     const uint32_t ta = tmem + (uint32_t(32 * (warp & 1)) << 16);
-    for (int b = b0; b < b1 && ok; ++b) {
-      const int i = b - b0;
-      ok = __all_sync(0xffffffffu, wait(done + (i & 1), uint32_t(i >> 1) & 1u));
+    for (int q = 0; q < (b1 - b0) * NSB; ++q) {
+      ok = __all_sync(0xffffffffu, wait(summed, uint32_t(q) & 1u));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
       if (32 * (warp & 1) < Cfg::ROWS) {
@@ -203,7 +212,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad_tc(const WgradArgs p) {
             float v[16];
             tmem_ld<16>(ta + uint32_t(c0), v);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) acc[c][e] += v[e];
+            for (int e = 0; e < 16; ++e) acc[c][e] = fmaf(v[e], 1.00000011920928955f, acc[c][e]);  // 1 + 2^-23
           }
         }
       }
@@ -217,30 +226,36 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad_tc(const WgradArgs p) {
     for (int b = b0; b < b1 && ok; ++b) {
       const int i = b - b0, buf = i & 1;
       ok = wait(full + buf, uint32_t(i >> 1) & 1u);
-      if (ok && i > 0) ok = wait(drained, uint32_t(i - 1) & 1u);
       if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;");
       const uint32_t og = uint32_t(buf * Cfg::BUF) >> 4, oa = og + uint32_t(Cfg::GB >> 4);
-      // smallest part first: the high part's 16 accumulations are then the only
-      // ones that round at the size of the sum
 #pragma unroll 1
-      for (int k = PA - 1; k >= 0; --k)
+      for (int h = 0; h < NSB; ++h) {
+        const int q = i * NSB + h;
+        if (q > 0 && !(ok = wait(drained, uint32_t(q - 1) & 1u))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        // smallest part first: the high part's accumulations are then the only
+        // ones that truncate at the size of the sum
 #pragma unroll 1
-        for (int yk = 0; yk < YB * (TX / 16); ++yk) {
-          const int yl = yk / (TX / 16), ks = yk % (TX / 16);
-          const uint64_t da = D0 + og + uint32_t(yl * GPL * (PLANE >> 4) + ks * 16);
+        for (int k = PA - 1; k >= 0; --k)
+#pragma unroll 1
+          for (int yk = 0; yk < SB * (TX / 16); ++yk) {
+            const int yl = h * SB + yk / (TX / 16), ks = yk % (TX / 16);
+            const uint64_t da = D0 + og + uint32_t(yl * GPL * (PLANE >> 4) + ks * 16);
 #pragma unroll
-          for (int dx = 0; dx < 3; ++dx) {
-            const uint64_t db = D0 + oa + uint32_t((k * (YB + 2) + yl) * CI * (PLANE >> 4) + ks * 16 + dx);
-            const uint32_t add = (yk > 0 || k < PA - 1) ? 1u : 0u;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "setp.ne.b32 p, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-                :
-                : "r"(tmem + uint32_t(dx * Cfg::NN)), "l"(da), "l"(db), "r"(IDESC), "r"(add));
+            for (int dx = 0; dx < 3; ++dx) {
+              const uint64_t db = D0 + oa + uint32_t((k * (YB + 2) + yl) * CI * (PLANE >> 4) + ks * 16 + dx);
+              const uint32_t add = (yk > 0 || k < PA - 1) ? 1u : 0u;
+              asm volatile(
+                  "{\n\t.reg .pred p;\n\t"
+                  "setp.ne.b32 p, %4, 0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+                  :
+                  : "r"(tmem + uint32_t(dx * Cfg::NN)), "l"(da), "l"(db), "r"(IDESC), "r"(add));
+            }
           }
-        }
+        mma_commit(summed);
+      }
+      // also after a wait that ran out: the exit waits for what was issued
       mma_commit(done + buf);
       last = b;
     }
