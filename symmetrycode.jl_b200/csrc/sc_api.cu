@@ -655,7 +655,8 @@ void tc_split_args(const sc_closure* cl, sc::CnnArgs& a) {
 // the BF16 roundings of weights and activations taken as identities.
 int tc_forward(sc_closure* cl, void* const* u, cudaStream_t st) {
   sc_plan* p = cl->p;
-  int rc = c2p_batch<float>(p, cl->bb, cl->cb, u, cl->gp, 3, st);
+  // the transform of closure_tauhat: the network is linearised at the activations it had there
+  int rc = c2p_batch<float>(p, cl->bb, cl->cb, u, cl->gp, 3, st, pinned(cl));
   if (rc) return rc;
   SC_CU(cudaMemsetAsync(cl->dsum, 0, sizeof(double), st));
   sc::launch_spectral_energy<float>(u, 3, 3, p->n, p->K1, p->K2, 1, p->kc, 2.0 * M_PI / p->l, 1, cl->dsum, st);
