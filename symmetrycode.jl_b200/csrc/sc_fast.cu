@@ -9,6 +9,7 @@ namespace sc {
 
 // the two-level split of the CTA-wide x sweeps
 template <int N> struct Split;
+template <> struct Split<810> { static constexpr int N1 = 27, N2 = 30; };
 template <> struct Split<128> { static constexpr int N1 = 16, N2 = 8; };
 template <> struct Split<64> { static constexpr int N1 = 8, N2 = 8; };
 
@@ -526,6 +527,7 @@ k_xsweep3(const XArgs a, const float2* __restrict__ tw) {
 // r2c: two-level register FFT per pencil, a pencil being one row of two
 // components packed as a + i b
 template <int N> struct XPF;
+template <> struct XPF<810> { static constexpr int TP = 8; };
 template <> struct XPF<128> { static constexpr int TP = 32; };
 template <> struct XPF<64> { static constexpr int TP = 32; };
 
@@ -727,7 +729,11 @@ template <int N> static void init_fast_n() {
     set_smem2(k_xsweep3<N>, X3Cfg<N>::SMEM);
     set_smem2(k_xr2c_fast<N>, XPFCfg<N>::SMEM);
   }
-  if (N == 810) set_smem2(k_xsweep4<true>, X4Cfg::SMEM), set_smem2(k_xsweep4<false>, X4Cfg::SMEM);
+  if constexpr (N == 810) {
+    set_smem2(k_xsweep4<true>, X4Cfg::SMEM);
+    set_smem2(k_xsweep4<false>, X4Cfg::SMEM);
+    set_smem2(k_xr2c_fast<N>, XPFCfg<N>::SMEM);
+  }
 }
 
 bool fast_supported(int N) { return N == 810 || N == 256 || N == 128 || N == 64; }
@@ -822,14 +828,33 @@ bool launch_xsweep3(int N, const XArgs& a, const void* tw, cudaStream_t st) {
 template <int N> static void xplain_n(bool inv, const XPlainArgs& a, const float2* t2, cudaStream_t st) {
   using Cfg = XPFCfg<N>;
   const long long npen = a.nrows * ((a.ncomp + 1) / 2);
-  if (inv) k_xc2r_warp<N><<<unsigned((npen + 7) / 8), 256, 0, st>>>(a, t2);
-  else k_xr2c_fast<N><<<unsigned((npen + Cfg::TP - 1) / Cfg::TP), Cfg::NT, Cfg::SMEM, st>>>(a, t2);
+  if constexpr (N <= 128) {
+    if (inv) {
+      k_xc2r_warp<N><<<unsigned((npen + 7) / 8), 256, 0, st>>>(a, t2);
+      return;
+    }
+  }
+  k_xr2c_fast<N><<<unsigned((npen + Cfg::TP - 1) / Cfg::TP), Cfg::NT, Cfg::SMEM, st>>>(a, t2);
 }
 
 bool launch_xplain_pinned(int N, bool inv, const XPlainArgs& a, const void* tw, cudaStream_t st) {
   const float2* t2 = static_cast<const float2*>(tw);
   if (N == 64) xplain_n<64>(inv, a, t2, st);
   else if (N == 128) xplain_n<128>(inv, a, t2, st);
+  else return false;
+  return true;
+}
+
+// One field of a 2D grid has so few rows that a transform's own length sets the
+// time, and where a row spread over more threads is there it is taken: c2r at 64
+// (to_phys of a 64^2 field 3.8 us, 4.2 with sc_xrow.cuh) and 128 (5.1, 5.9), r2c at
+// 810 (to_spec of an 810^2 field 11.9 us, 16.8).
+bool launch_xplain_one2d(int N, bool inv, const XPlainArgs& a, const void* tw, cudaStream_t st) {
+  if (a.ncomp != 1 || a.nrows != N) return false;
+  const float2* t2 = static_cast<const float2*>(tw);
+  if (inv && N == 64) xplain_n<64>(true, a, t2, st);
+  else if (inv && N == 128) xplain_n<128>(true, a, t2, st);
+  else if (!inv && N == 810) xplain_n<810>(false, a, t2, st);
   else return false;
   return true;
 }

@@ -153,6 +153,8 @@ bool launch_col2(int N, bool inv, const ColArgs& a, const void* tw, cudaStream_t
 // the x sweeps around the one-pass BF16 closure network, N = 64 and 128 (sc_fast.cu)
 bool launch_xsweep3(int N, const XArgs& a, const void* tw, cudaStream_t st);
 bool launch_xplain_pinned(int N, bool inv, const XPlainArgs& a, const void* tw, cudaStream_t st);
+// FP32 transforms of one 2D field that other kernels than sc_xrow.cuh's do faster
+bool launch_xplain_one2d(int N, bool inv, const XPlainArgs& a, const void* tw, cudaStream_t st);
 // 3D product sweep of N = 810 (false: the variant is the general sweep of sc_xrow.h)
 bool launch_xsweep810(const XArgs& a, const void* tw, cudaStream_t st);
 // randomfield on the device (sc_random.cu): counter-based N(0, 1/2) draws into

@@ -909,6 +909,7 @@ template <typename R> bool launch_xsweep_ns(int N, const XArgs& a, const void* t
 }
 template <typename R> bool launch_x_c2r(int N, const XPlainArgs& a, const void* tw, cudaStream_t st) {
   if (sizeof(R) == 4 && a.pinned && launch_xplain_pinned(N, true, a, tw, st)) return true;
+  if (sizeof(R) == 4 && launch_xplain_one2d(N, true, a, tw, st)) return true;
   if (xrow_c2r<R>(N, a, tw, st)) return true;
   switch (N) {
 #define SC_CASE(NN) case NN: return xc2r_n<R, NN>(a, tw, st);
@@ -922,6 +923,7 @@ template <typename R> bool launch_x_point(int N, const XPointArgs& a, const void
 }
 template <typename R> bool launch_x_r2c(int N, const XPlainArgs& a, const void* tw, cudaStream_t st) {
   if (sizeof(R) == 4 && a.pinned && launch_xplain_pinned(N, false, a, tw, st)) return true;
+  if (sizeof(R) == 4 && launch_xplain_one2d(N, false, a, tw, st)) return true;
   if (xrow_r2c<R>(N, a, tw, st)) return true;
   switch (N) {
 #define SC_CASE(NN) case NN: return xr2c_n<R, NN>(a, tw, st);
