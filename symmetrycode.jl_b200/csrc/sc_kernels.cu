@@ -896,7 +896,7 @@ template <typename R> bool launch_col_fwd(int N, const ColArgs& a, const void* t
     default: return false;
   }
 }
-template <typename R> bool launch_xsweep_ns(int N, const XArgs& a, const void* tw, cudaStream_t st) {
+template <typename R> static bool xsweep_ns(int N, const XArgs& a, const void* tw, cudaStream_t st) {
   if (sizeof(R) == 4 && launch_xsweep3(N, a, tw, st)) return true;
   if (sizeof(R) == 4 && N == 810 && launch_xsweep810(a, tw, st)) return true;
   if (xrow_ns<R>(N, a, tw, st)) return true;
@@ -906,6 +906,19 @@ template <typename R> bool launch_xsweep_ns(int N, const XArgs& a, const void* t
 #undef SC_CASE
     default: return false;
   }
+}
+template <typename R> bool launch_xsweep_ns(int N, const XArgs& a, const void* tw, cudaStream_t st) {
+  using C = typename V2<R>::T;
+  const int ldo = a.ldo > 0 ? a.ldo : a.K1out;
+  const long long step = sweep_rows(a.K1in > ldo ? a.K1in : ldo);
+  XArgs b = a;
+  for (long long r = 0; r < a.nrows; r += step) {
+    b.nrows = a.nrows - r < step ? a.nrows - r : step;
+    for (int c = 0; c < a.D; ++c) b.in[c] = static_cast<const C*>(a.in[c]) + r * a.K1in;
+    for (int c = 0; c < (a.D == 3 ? 6 : 3); ++c) b.out[c] = static_cast<C*>(a.out[c]) + r * ldo;
+    if (!xsweep_ns<R>(N, b, tw, st)) return false;
+  }
+  return true;
 }
 template <typename R> bool launch_x_c2r(int N, const XPlainArgs& a, const void* tw, cudaStream_t st) {
   if (sizeof(R) == 4 && a.pinned && launch_xplain_pinned(N, true, a, tw, st)) return true;

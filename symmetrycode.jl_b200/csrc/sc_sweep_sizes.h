@@ -63,6 +63,12 @@ inline bool sweep_size(int n, bool f32, int* xn1 = nullptr, int* xn2 = nullptr) 
   }
 }
 
+// Rows of one launch of a product sweep whose rows are `len` elements long: whole
+// row pairs, and few enough that the kernels' 32-bit element indexes (those of a last
+// warp that is partly empty included) stay below 2^31.  A plan's n^2 rows always are
+// (n <= 1024); the microbenchmark takes any number.
+inline long long sweep_rows(long long len) { return (2147483647LL / len - 64) & ~1LL; }
+
 // the smallest of these sizes that is at least m (0: none)
 inline int sweep_size_from(int m) {
 #define SC_CASE(N, ...) if (N >= m) return N;
