@@ -1636,9 +1636,10 @@ int sc_closure_create(sc_closure** out, sc_plan* p, int kind, double delta, cons
     if (!rc && table) {
       const double width = kind == sc::kBardina ? cl->prm[0] * delta : 2.0 * delta, kfac = 2.0 * M_PI / p->l;
       cl->wtab = cl->dsum + 256 / sizeof(double);
-      if (p->dtype == SC_FLOAT64) sc::launch_gauss_table<double>(cl->wtab, nq, kfac, width, 0);
-      else sc::launch_gauss_table<float>(cl->wtab, nq, kfac, width, 0);
-      if (cudaStreamSynchronize(0) != cudaSuccess) rc = fail(SC_ERR_CUDA, "test filter table");
+      // on the plan's own stream: not behind the work that the caller has queued
+      if (p->dtype == SC_FLOAT64) sc::launch_gauss_table<double>(cl->wtab, nq, kfac, width, p->cap);
+      else sc::launch_gauss_table<float>(cl->wtab, nq, kfac, width, p->cap);
+      if (cudaStreamSynchronize(p->cap) != cudaSuccess) rc = fail(SC_ERR_CUDA, "test filter table");
     }
   }
   if (rc) {
