@@ -9,8 +9,8 @@ x-sweep kernel (``sc_plan_num_variants``).  ``tune`` times every variant of
 every sweep on the plan's own buffers with CUDA events
 (``sc_state_profile_rhs``, one right-hand side of the plan's state per
 repetition), keeps the fastest per sweep (``sc_plan_set_option``) and records
-the choice and the timings in a JSON cache keyed by device, grid and
-precision, so later plans of the same shape reuse it without timing.
+the choice and the timings in a JSON cache keyed by device, grid, precision
+and kernel set, so later plans of the same shape reuse it without timing.
 
 Usage::
 
@@ -64,8 +64,13 @@ def choose(timings, counts):
     return best
 
 
+# raised whenever a variant number comes to mean another kernel, so that a choice
+# stored by an earlier build is timed again (2: the x sweeps of 64, 128 and 810)
+KERNEL_SET = 2
+
+
 def cache_key(device_name, D, n, dtype_name):
-    return f"{device_name}|D={D}|n={n}|{dtype_name}"
+    return f"{device_name}|D={D}|n={n}|{dtype_name}|kernels={KERNEL_SET}"
 
 
 def default_cache_path():
