@@ -2662,6 +2662,8 @@ int sc_plan_set_option(sc_plan* p, int option, long long value) {
     const int sweep = option - SC_OPT_VARIANT_ZINV;
     int nv = 0;
     sc_plan_num_variants(p, sweep, &nv);
+    // 256 once had a second x sweep: its number, in a caller's saved choice, is the default
+    if (sweep == 2 && p->n == 256 && p->D == 3 && p->dtype == SC_FLOAT32 && value == 1) value = 0;
     if (value < 0 || value >= nv) return fail(SC_ERR_INVALID, "sweep %d has %d variants", sweep, nv);
     p->variant[sweep] = int(value);
     // cached step graphs hold the old launches

@@ -805,10 +805,10 @@ int col2_variants(int N) {
 // for its twiddles), 3 = the warp-per-row-pair sweep of the other sizes (1096
 // us: a warp of 30 x 27 points holds too many registers to keep the issue slots
 // busy).  At 64 and 128, 0 = the warp-per-row-pair sweep and 1 = the CTA-wide
-// sweep above; 256 has the first only and takes 1 for it too.
+// sweep above; 256 has the first only.
 int xsweep_variants(int N, int D) {
-  if (D != 3 || !fast_supported(N)) return 1;
-  return N == 810 ? 4 : 2;
+  if (D != 3) return 1;
+  return N == 810 ? 4 : N == 64 || N == 128 ? 2 : 1;
 }
 
 template <int N> static void xsweep3_n(const XArgs& a, const float2* t2, cudaStream_t st) {
