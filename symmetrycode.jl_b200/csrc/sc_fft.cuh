@@ -1,4 +1,4 @@
-// Register DFTs of radix 2 to 45, and the mixed-radix (2, 3, 5) FFT engine for a
+// Register DFTs of radix 2 to 32, and the mixed-radix (2, 3, 5) FFT engine for a
 // tile of pencils held in shared memory (sizes below 32).
 //
 // The spectral transforms of the solver stand in for the cuFFT/FFTW `plan_rfft`
@@ -233,13 +233,9 @@ template <bool INV, typename C> struct DFT<16, INV, C> : DFTPQ<4, 4, INV, C> {};
 template <bool INV, typename C> struct DFT<18, INV, C> : DFTPFA<2, 9, INV, C> {};
 template <bool INV, typename C> struct DFT<20, INV, C> : DFTPFA<4, 5, INV, C> {};
 template <bool INV, typename C> struct DFT<24, INV, C> : DFTPFA<8, 3, INV, C> {};
-template <bool INV, typename C> struct DFT<25, INV, C> : DFTPQ<5, 5, INV, C> {};
 template <bool INV, typename C> struct DFT<27, INV, C> : DFTPQ<3, 9, INV, C> {};
 template <bool INV, typename C> struct DFT<30, INV, C> : DFTPFA<3, 10, INV, C> {};
 template <bool INV, typename C> struct DFT<32, INV, C> : DFTPQ<4, 8, INV, C> {};
-template <bool INV, typename C> struct DFT<36, INV, C> : DFTPFA<4, 9, INV, C> {};
-template <bool INV, typename C> struct DFT<40, INV, C> : DFTPFA<8, 5, INV, C> {};
-template <bool INV, typename C> struct DFT<45, INV, C> : DFTPFA<5, 9, INV, C> {};
 
 // ---------------------------------------------------------------------------
 // radix schedule for N = 2^a 3^b 5^c (compile time)
