@@ -197,6 +197,11 @@ int plan_alloc(sc_plan* p, void** out, size_t bytes) {
 // sweep.  Taken when at least a tenth of the points per axis go (256 -> 128 would
 // leave 240: no faster, and a radix-5 size rounds a little more than a power of
 // two).  0: the DNS grid, also where the x sweep does not take the shape.
+// Accuracy, FP32: tau is the small difference of two product spectra.  Rounded
+// constants (1 / M^3 and those of the DFTs) leave a common factor of 1e-8 to 2e-7 in
+// each, another for every size, and whether the two cancel is a matter of the pair of
+// sizes.  Over 33 pairs at three widths tau's error is 0.70 to 1.71 times that on the
+// DNS grid, 1.04 in the geometric mean (810 -> 128: 1.13, 1.10, 1.02).
 int reduced_grid(const sc_plan* p, int kout) {
   const int m = sc::sweep_size_from(2 * p->kc + kout + 1);
   return p->D == 3 && m > 0 && 10 * m <= 9 * p->n && p->kc > m / 3 && kout <= m / 5 ? m : 0;

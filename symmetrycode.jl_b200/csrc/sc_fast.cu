@@ -347,8 +347,9 @@ k_xsweep4(const XArgs a, const float2* __restrict__ tw) {
 // input into a difference of the size of the roundings themselves: the sweeps
 // of sc_xrow.cuh, equally exact, moved the state of a 128^3 step by 1.9e-5
 // where the network's own error is 3.9e-5.  So the transforms of a right-hand
-// side with that network keep these kernels and with them, bit for bit, the
-// results of earlier runs; they cost 70 us of a 2.9 ms step.
+// side with that network, and of its adjoint, keep these kernels and with them,
+// bit for bit, the results of earlier runs (on a plan whose column sweeps are the
+// default ones); they cost 70 us of a 2.9 ms step.
 //
 // Product sweep, rows paired: u3 of rows 2q and 2q+1 share one inverse transform
 // (1.5 inverse transforms per row instead of 2) and the forward side runs in two

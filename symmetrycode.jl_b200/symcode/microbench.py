@@ -17,8 +17,8 @@ at n^3 (FP32).
 ``--kernel cnn`` evaluates the tensor-core CNN closure (n = 128, FP32) COUNT
 times on a seeded random field and reports ms per evaluation and the
 convolutions' TFLOP/s (2 x 27 x sum(C_in C_out) flops per grid point);
-``--split`` in split precision (three passes per convolution; the TFLOP/s
-count one pass's flops).
+``--split`` in split precision (three products per convolution; the TFLOP/s
+count one product's flops).
 
 ``--kernel adjoint`` runs one a-posteriori training rollout of the tensor-core
 CNN closure at n^3 (default n = 64 with ``--n 64``): record a target
